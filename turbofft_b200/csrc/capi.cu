@@ -323,6 +323,22 @@ int ilog2_exact(long long x) {
 // a launch can repair from the running checksums if the kernel exists and its three tiles fit
 bool csum_ok(const KernelEntry* k) { return k && k->fn[FT_CSUM] && k->smem_csum <= 227u * 1024u; }
 
+// Launches one fft_kernel with the programmatic-dependent-launch attribute (fft_kernels.cuh,
+// wait_for_previous_launch): its blocks are placed while the launch before it drains.
+cudaError_t launch_kernel(const void* fn, unsigned grid, int threads, void** args, size_t smem, cudaStream_t st) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 template <typename T>
 int launch_cluster(tfft_plan p, const void* in, void* out, cudaStream_t st) {
     typedef typename Cplx<T>::type C;
@@ -453,7 +469,7 @@ int launch_all(tfft_plan p, const void* in, void* out, cudaStream_t st, void* sc
         const bool use_csum = ftmode == FT_CORRECT && p->csum && csum_ok(d.k);
         const void* fn = use_csum ? d.k->fn[FT_CSUM] : d.k->fn[ftmode];
         const size_t smem = use_csum ? d.k->smem_csum : d.k->smem;
-        if (!cuda_ok(p, cudaLaunchKernel(fn, dim3(d.grid), dim3(d.k->threads), args, smem, st)))
+        if (!cuda_ok(p, launch_kernel(fn, d.grid, d.k->threads, args, smem, st)))
             return TFFT_ERR_CUDA;
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }
@@ -1320,7 +1336,7 @@ int static_launch(const StaticDeviceState& st, int logN, const void* in, void* o
         a.tw_lo_bits = d.tw_lo_bits;
         a.inj_period = 1;
         void* args[] = {&a};
-        if (cudaLaunchKernel(d.k->fn[FT_OFF], dim3(d.grid), dim3(d.k->threads), args, d.k->smem, stream) != cudaSuccess)
+        if (launch_kernel(d.k->fn[FT_OFF], d.grid, d.k->threads, args, d.k->smem, stream) != cudaSuccess)
             return TFFT_ERR_CUDA;
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }

@@ -141,6 +141,18 @@ __device__ __forceinline__ float acc_sum(float2 acc) { return acc.x + acc.y; }
 template <> __device__ __forceinline__ float2 acc_zero<float2>() { return make_float2(0.0f, 0.0f); }
 #endif
 
+// Programmatic dependent launch.  No block touches global data before the launch before it has completed and its
+// stores are visible (wait_for_previous_launch); once every block has got as far as the stores of its first tile, the
+// next launch of the stream may place its blocks in the slots that this one's tail leaves empty (let_next_launch_start).
+// Every block waits, so completion is transitive: whoever waits for this launch has waited for all earlier ones.
+// Without the launch attribute (launch_kernel in capi.cu) both instructions do nothing.
+// Bound: launch latency and the drain between two launches.  Measured back to back on one stream, before -> after:
+// 2^16 x 1 10.9 -> 6.0 us, 2^22 x 1 41 -> 34 us, 2^16 x 512 175 -> 170 us (complex64).  The start signal stands before
+// the stores because a launch placed earlier finds the SMs still occupied and is spread unevenly: with the signal at
+// the top of the kernel 2^16 x 8 takes 9.6 us, here 7.1 us.
+__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+
 // cos(2*pi*k/32), k = 0..8
 template <typename T> __device__ __forceinline__ constexpr T cos32_tab(int k) {
     return k == 0 ? T(1.0)
@@ -488,6 +500,7 @@ struct Fft {
                 y[i].y *= a.scale_y;
             }
         }
+        let_next_launch_start();
         if constexpr (K::STAGED_IO) {
             // every thread only touches its own line here, so no barrier is needed before
 #pragma unroll
@@ -787,6 +800,7 @@ __global__ void __launch_bounds__((Cfg<T, LOGM, LOGE, LOGC, ROLE>::THREADS),
 fft_kernel(const __grid_constant__ KernelArgs<T> a) {
     extern __shared__ __align__(16) unsigned char tfft_smem_raw[];
     typedef typename Cplx<T>::type C;
+    wait_for_previous_launch();
     Fft<T, LOGM, LOGE, LOGC, ROLE, FT>::run(a, reinterpret_cast<C*>(tfft_smem_raw));
 }
 
