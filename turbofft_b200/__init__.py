@@ -83,6 +83,9 @@ class Plan:
 
     def __call__(self, x, out=None):
         """x: CUDA tensor [batch, N] (or [N] when batch == 1) of the plan's dtype."""
+        y = (_binding or _load_binding()).exec(self, x, out)
+        if y is not None:
+            return y
         torch = _torch()
         if not x.is_cuda:
             raise ValueError("input must be a CUDA tensor (use exec_host for host buffers)")
@@ -107,9 +110,7 @@ class Plan:
         x = x.contiguous()
         if out is None:
             out = torch.empty_like(x, pin_memory=x.is_pinned())
-        with torch.cuda.device(self.device):
-            stream = torch.cuda.current_stream().cuda_stream
-            self.exec_host_ptr(x.data_ptr(), out.data_ptr(), stream)
+        self.exec_host_ptr(x.data_ptr(), out.data_ptr(), torch.cuda.current_stream(self.device).cuda_stream)
         return out
 
     def exec_host_async(self, x, out):
@@ -120,9 +121,7 @@ class Plan:
         if x.is_cuda or out.is_cuda or _dtype_code(x.dtype) != self.dtype or x.numel() != self.batch << self.logN \
                 or out.dtype != x.dtype or out.numel() != x.numel() or not (x.is_contiguous() and out.is_contiguous()):
             raise ValueError("tensors do not match the plan")
-        with torch.cuda.device(self.device):
-            stream = torch.cuda.current_stream().cuda_stream
-            self.exec_host_async_ptr(x.data_ptr(), out.data_ptr(), stream)
+        self.exec_host_async_ptr(x.data_ptr(), out.data_ptr(), torch.cuda.current_stream(self.device).cuda_stream)
         return out
 
     # -- introspection
@@ -160,13 +159,10 @@ class Plan:
 
     def ft_status(self, launch: int = -1):
         """(n_detected, n_corrected, located[list per block of `launch`])."""
-        nd, nc, nb = C.c_int(), C.c_int(), C.c_int()
-        _lib.check(lib().tfft_ft_status(self._h, C.byref(nd), C.byref(nc), launch, None, 0, C.byref(nb)),
-                   "tfft_ft_status", self._h)
-        loc = (C.c_int * max(nb.value, 1))()
-        _lib.check(lib().tfft_ft_status(self._h, C.byref(nd), C.byref(nc), launch, loc, nb.value, C.byref(nb)),
-                   "tfft_ft_status", self._h)
-        return nd.value, nc.value, list(loc[: nb.value])
+        status = (_binding or _load_binding()).ft_status(self, int(launch))
+        if isinstance(status, int):
+            _lib.check(status, "tfft_ft_status", self._h)
+        return status
 
     def ft_diag(self, launch: int = -1):
         """Per block (delta, S, delta_w) of `launch`; needs enable_ft_diag() before exec."""
@@ -188,6 +184,20 @@ class Plan:
 
 
 _plan_cache = {}
+_binding = None
+
+
+def _load_binding():
+    """The native call path (csrc/torch_binding.cpp), bound to the loaded library and the plan cache; it
+    answers None to whatever is not an ordinary call, which the Python code then handles."""
+    global _binding
+    _torch()  # the module's libtorch symbols
+    from . import _torch_binding
+
+    entry = [C.cast(f, C.c_void_p).value for f in (lib().tfft_exec, lib().tfft_ft_status, lib().tfft_plan_info)]
+    _torch_binding.bind(*entry, _plan_cache)
+    _binding = _torch_binding
+    return _binding
 
 
 _NORM_FWD = {None: 0.0, "backward": 0.0, "ortho": -0.5, "forward": -1.0}  # exponent of N in the forward scale
@@ -233,6 +243,11 @@ def fft(x, ft: bool = False, err: bool = False, thread_bs: int = 1, out=None, no
     (no copy, no transpose; lengths with a compiled strided-line kernel, FT off).  Plans are
     cached per (device, shape, mode).
     """
+    expo = _NORM_FWD.get(norm)
+    if expo is not None:
+        y = (_binding or _load_binding()).fft(x, ft, err, thread_bs, out, -1.0 - expo if inverse else expo, inverse, dim)
+        if y is not None:
+            return y
     if not x.is_cuda:
         raise ValueError("turbofft_b200.fft needs a CUDA tensor: there is no CPU path")
     if norm not in _NORM_FWD:

@@ -127,7 +127,8 @@ struct tfft_plan_s {
     void* scratch = nullptr;
     void* scratch2 = nullptr;          // 3-launch plans that correct: the middle launch writes here, so that
                                        // its own input survives for the recompute of a located tile
-    unsigned int* ft_count = nullptr;  // [3][2]
+    unsigned int* ft_count = nullptr;  // [3][2], counted only while ft_accumulate is set
+    int* ft_located = nullptr;         // the per-block results of all launches, one after the other
     unsigned long long* oob = nullptr;  // checked build: first out-of-range access of the last exec
     size_t owned_bytes = 0;
     double err_inj = TFFT_DEFAULT_ERR_INJ;
@@ -323,6 +324,31 @@ int ilog2_exact(long long x) {
 // a launch can repair from the running checksums if the kernel exists and its three tiles fit
 bool csum_ok(const KernelEntry* k) { return k && k->fn[FT_CSUM] && k->smem_csum <= 227u * 1024u; }
 
+// blocks of all launches: entries of tfft_plan_s::ft_located
+size_t ft_blocks(tfft_plan p) {
+    size_t n = 0;
+    for (int i = 0; i < p->n_launch; ++i) n += p->L[i].grid;
+    return n;
+}
+
+// Detected blocks and repaired tiles of launch i, from its per-block results.  A block repairs the tile it located
+// if it worked through that many (fft_kernels.cuh, Fft::run); only plans that correct do.
+void count_located(tfft_plan p, int i, const int* located, long long& detected, long long& repaired) {
+    const LaunchDesc& d = p->L[i];
+    for (long long b = 0; b < d.grid; ++b) {
+        const int k = located[b];
+        if (k == -1) continue;
+        ++detected;
+        if (p->if_err && k >= 1 && k <= p->thread_bs && b + (k - 1) * (long long)d.grid < d.n_tiles) ++repaired;
+    }
+}
+
+// Pinned landing place of tfft_ft_status: a copy into pageable memory is staged by the driver and waits on its own.
+// One for all plans, made at the first call; longer results take the pageable route.
+constexpr size_t kStatusBytes = 64u << 10;
+std::mutex g_status_mu;
+int* g_status_host = nullptr;
+
 // Launches one fft_kernel with the programmatic-dependent-launch attribute (fft_kernels.cuh,
 // wait_for_previous_launch): its blocks are placed while the launch before it drains.
 cudaError_t launch_kernel(const void* fn, unsigned grid, int threads, void** args, size_t smem, cudaStream_t st) {
@@ -422,9 +448,6 @@ int launch_all(tfft_plan p, const void* in, void* out, cudaStream_t st, void* sc
     if (p->ck) return launch_cluster<T>(p, in, out, st);
     if (p->pk) return launch_pair<T>(p, in, out, st);
     const int ftmode = p->if_ft ? (p->if_err ? FT_CORRECT : FT_DETECT) : FT_OFF;
-    if (p->if_ft && !p->ft_accumulate) {
-        if (!cuda_ok(p, cudaMemsetAsync(p->ft_count, 0, 6 * sizeof(unsigned int), st))) return TFFT_ERR_CUDA;
-    }
     const int inj_launch = p->inj_launch < 0 ? p->n_launch - 1 : p->inj_launch;
     for (int i = 0; i < p->n_launch; ++i) {
         const LaunchDesc& d = p->L[i];
@@ -463,7 +486,7 @@ int launch_all(tfft_plan p, const void* in, void* out, cudaStream_t st, void* sc
         a.n_elems = p->batch << p->logn;
         a.oob = p->oob;
         a.ft_located = d.ft_located;
-        a.ft_count = p->ft_count ? p->ft_count + 2 * i : nullptr;
+        a.ft_count = p->ft_accumulate ? p->ft_count + 2 * i : nullptr;
         a.ft_diag = p->diag ? (T*)d.ft_diag : nullptr;
         void* args[] = {&a};
         const bool use_csum = ftmode == FT_CORRECT && p->csum && csum_ok(d.k);
@@ -617,12 +640,18 @@ int tfft_plan_create(tfft_plan* plan, int logN, long long batch, int dtype, int 
 #endif
     if (status == TFFT_OK && p->if_ft) {
         p->ft_count = (unsigned int*)dev_alloc(p, 6 * sizeof(unsigned int));
-        // zeroed here as well as before every exec: in accumulating mode nothing else clears them
-        if (!p->ft_count || !cuda_ok(p, cudaMemset(p->ft_count, 0, 6 * sizeof(unsigned int)))) status = TFFT_ERR_ALLOC;
+        const size_t blocks = ft_blocks(p);
+        p->ft_located = (int*)dev_alloc(p, blocks * sizeof(int));
+        // tfft_ft_status before the first exec finds nothing detected
+        if (!p->ft_count || !p->ft_located || !cuda_ok(p, cudaMemset(p->ft_count, 0, 6 * sizeof(unsigned int))) ||
+            !cuda_ok(p, cudaMemset(p->ft_located, 0xff, blocks * sizeof(int))))
+            status = TFFT_ERR_ALLOC;
+        size_t at = 0;
         for (int i = 0; i < p->n_launch && status == TFFT_OK; ++i) {
-            p->L[i].ft_located = (int*)dev_alloc(p, (size_t)p->L[i].grid * sizeof(int));
+            p->L[i].ft_located = p->ft_located + at;
+            at += p->L[i].grid;
             p->L[i].ft_diag = dev_alloc(p, (size_t)p->L[i].grid * 3 * (p->esize() / 2));
-            if (!p->L[i].ft_located || !p->L[i].ft_diag) status = TFFT_ERR_ALLOC;
+            if (!p->L[i].ft_diag) status = TFFT_ERR_ALLOC;
         }
     }
     if (status != TFFT_OK) {
@@ -1074,22 +1103,45 @@ int tfft_ft_status(tfft_plan p, int* n_detected, int* n_corrected, int launch, i
     if (!p->if_ft) return TFFT_OK;
     DeviceGuard guard(p->device);
     if (!guard.ok) return TFFT_ERR_CUDA;
-    if (!cuda_ok(p, cudaStreamSynchronize(p->last_stream))) return TFFT_ERR_CUDA;
-    unsigned int cnt[6];
-    if (!cuda_ok(p, cudaMemcpy(cnt, p->ft_count, sizeof(cnt), cudaMemcpyDeviceToHost))) return TFFT_ERR_CUDA;
-    if (p->ft_accumulate && !cuda_ok(p, cudaMemset(p->ft_count, 0, sizeof(cnt)))) return TFFT_ERR_CUDA;
-    for (int i = 0; i < p->n_launch; ++i) {
-        if (n_detected) *n_detected += (int)cnt[2 * i];
-        if (n_corrected) *n_corrected += (int)cnt[2 * i + 1];
-    }
     if (launch < 0) launch = p->n_launch - 1;
     if (launch >= p->n_launch) return TFFT_ERR_BAD_ARG;
-    if (n_blocks) *n_blocks = (int)p->L[launch].grid;
-    if (located && cap > 0) {
-        const size_t n = (size_t)(cap < (int)p->L[launch].grid ? cap : (int)p->L[launch].grid);
-        if (!cuda_ok(p, cudaMemcpy(located, p->L[launch].ft_located, n * sizeof(int), cudaMemcpyDeviceToHost)))
-            return TFFT_ERR_CUDA;
+    // One copy and one wait: the per-block results say which blocks detected and which tiles were repaired, so an
+    // exec neither clears nor counts anything.  (Counters cleared by a memset before every exec, a wait and a copy
+    // each for counters and blocks: 286 us for exec + status of 2^12 x 2^14 complex64 became 245 us.)
+    const size_t blocks = ft_blocks(p), bytes = blocks * sizeof(int);
+    std::vector<int> pageable;
+    std::unique_lock<std::mutex> lock(g_status_mu);
+    if (!g_status_host && !cuda_ok(p, cudaHostAlloc((void**)&g_status_host, kStatusBytes, cudaHostAllocPortable))) return TFFT_ERR_CUDA;
+    int* host = g_status_host;
+    if (bytes > kStatusBytes) {
+        lock.unlock();
+        pageable.resize(blocks);
+        host = pageable.data();
     }
+    if (!cuda_ok(p, cudaMemcpyAsync(host, p->ft_located, bytes, cudaMemcpyDeviceToHost, p->last_stream)) ||
+        !cuda_ok(p, cudaStreamSynchronize(p->last_stream)))
+        return TFFT_ERR_CUDA;
+    long long detected = 0, repaired = 0;
+    if (p->ft_accumulate) {
+        unsigned int cnt[6];
+        if (!cuda_ok(p, cudaMemcpy(cnt, p->ft_count, sizeof(cnt), cudaMemcpyDeviceToHost)) ||
+            !cuda_ok(p, cudaMemset(p->ft_count, 0, sizeof(cnt))))
+            return TFFT_ERR_CUDA;
+        for (int i = 0; i < p->n_launch; ++i) {
+            detected += cnt[2 * i];
+            repaired += cnt[2 * i + 1];
+        }
+    }
+    const int* l = host;
+    for (int i = 0; i < p->n_launch; ++i) {
+        if (!p->ft_accumulate) count_located(p, i, l, detected, repaired);
+        if (i == launch && located && cap > 0)
+            memcpy(located, l, (size_t)(cap < (int)p->L[i].grid ? cap : (int)p->L[i].grid) * sizeof(int));
+        l += p->L[i].grid;
+    }
+    if (n_detected) *n_detected = (int)detected;
+    if (n_corrected) *n_corrected = (int)repaired;
+    if (n_blocks) *n_blocks = (int)p->L[launch].grid;
     return TFFT_OK;
 }
 

@@ -1,0 +1,251 @@
+// CPython face of the call path a program takes once per transform: turbofft_b200.fft / ifft,
+// Plan.__call__ on ordinary CUDA tensors, Plan.ft_status.
+//
+// A 16 x 1024-point transform keeps the GPU busy for 2.5 us; the interpreted form of this path
+// (attribute reads, a key tuple, reshape, ctypes argument conversion) kept the caller busy for 15.
+// Here a call reads the tensor's fields through ATen, looks the plan up in the SAME dictionary the
+// Python side keeps, allocates the output and calls tfft_exec.  Whatever is not an ordinary call --
+// a plan that does not exist yet, a tensor that is not on a GPU, not contiguous, of
+// another type or length -- returns None, and the Python code does what it always did, errors included.
+// The module links nothing of the library: it is handed the address of the tfft_exec that _lib.py loaded.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cstdint>
+#include <vector>
+
+namespace {
+
+typedef int (*ExecFn)(void*, const void*, void*, void*);
+typedef int (*StatusFn)(void*, int*, int*, int, int*, int, int*);
+typedef int (*InfoFn)(void*, int*);
+
+ExecFn g_exec = nullptr;
+StatusFn g_status = nullptr;
+InfoFn g_info = nullptr;
+PyObject* g_plans = nullptr;  // turbofft_b200._plan_cache
+PyObject *s_h, *s_value, *s_logn, *s_batch, *s_dtype, *s_device, *s_strided;
+
+// complex64 -> 0, complex128 -> 1 (the C ABI's dtype codes), anything else -> -1
+int type_code(const at::Tensor& x) {
+    const auto t = x.scalar_type();
+    return t == at::kComplexFloat ? 0 : (t == at::kComplexDouble ? 1 : -1);
+}
+
+bool ordinary(PyObject* o) { return THPVariable_CheckExact(o); }
+
+// an int attribute of a Plan; false (no error set) if it is not one
+bool int_attr(PyObject* o, PyObject* name, long long* v) {
+    PyObject* a = PyObject_GetAttr(o, name);
+    if (!a) {
+        PyErr_Clear();
+        return false;
+    }
+    *v = PyLong_Check(a) ? PyLong_AsLongLong(a) : -1;
+    Py_DECREF(a);
+    if (PyErr_Occurred()) {
+        PyErr_Clear();
+        return false;
+    }
+    return true;
+}
+
+// the tfft_plan behind a Plan object, null for a destroyed one
+void* plan_handle(PyObject* plan) {
+    PyObject* h = PyObject_GetAttr(plan, s_h);
+    PyObject* v = h ? PyObject_GetAttr(h, s_value) : nullptr;
+    void* p = v && PyLong_Check(v) ? PyLong_AsVoidPtr(v) : nullptr;
+    Py_XDECREF(v);
+    Py_XDECREF(h);
+    if (PyErr_Occurred()) PyErr_Clear();
+    return p;
+}
+
+// Allocates the output (unless the caller brought one) and runs the plan on the current stream of the
+// tensor's device.  None when the library reports an error: the Python path repeats the call and raises.
+PyObject* execute(void* plan, const at::Tensor& x, PyObject* out_obj) {
+    at::Tensor y;
+    if (out_obj == Py_None) y = at::empty(x.sizes(), x.options());
+    else y = THPVariable_Unpack(out_obj);
+    void* stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+    int rc;
+    const void* in = x.const_data_ptr();
+    void* out = y.mutable_data_ptr();
+    Py_BEGIN_ALLOW_THREADS
+    rc = g_exec(plan, in, out, stream);
+    Py_END_ALLOW_THREADS
+    if (rc != 0) Py_RETURN_NONE;
+    if (out_obj != Py_None) {
+        Py_INCREF(out_obj);
+        return out_obj;
+    }
+    return THPVariable_Wrap(std::move(y));
+}
+
+// fft(x, ft, err, thread_bs, out, norm_exponent, inverse, dim): the transform along one axis, or None
+PyObject* fast_fft(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 8 || !g_exec || !ordinary(a[0]) || !PyLong_Check(a[7])) Py_RETURN_NONE;
+    try {
+        const at::Tensor& x = THPVariable_Unpack(a[0]);
+        const int code = type_code(x);
+        const int64_t rank = x.dim();
+        int64_t dim = PyLong_AsLong(a[7]);
+        if (dim < 0) dim += rank;
+        if (code < 0 || !x.is_cuda() || dim < 0 || dim >= rank || x.numel() == 0 || !x.is_contiguous()) Py_RETURN_NONE;
+        const int64_t len = x.size(dim);
+        if (len < 2 || (len & (len - 1))) Py_RETURN_NONE;
+        const int logn = __builtin_ctzll((unsigned long long)len);
+        if (a[4] != Py_None) {
+            if (!ordinary(a[4])) Py_RETURN_NONE;
+            const at::Tensor& y = THPVariable_Unpack(a[4]);
+            if (!y.is_cuda() || !y.is_contiguous() || y.scalar_type() != x.scalar_type() || y.sizes() != x.sizes()) Py_RETURN_NONE;
+        }
+        const int ft = PyObject_IsTrue(a[1]), err = PyObject_IsTrue(a[2]), inverse = PyObject_IsTrue(a[6]);
+        if (ft < 0 || err < 0 || inverse < 0) return nullptr;
+        // the keys turbofft_b200.fft files its plans under
+        const bool strided = dim != rank - 1;
+        if (strided && (ft || err || a[4] != Py_None)) Py_RETURN_NONE;
+        PyObject* key = PyTuple_New(strided ? 8 : 9);
+        if (!key) return nullptr;
+        int k = 0;
+        auto put = [&](PyObject* o) { PyTuple_SET_ITEM(key, k++, o); };
+        auto put_ref = [&](PyObject* o) {
+            Py_INCREF(o);
+            put(o);
+        };
+        if (strided) {
+            int64_t inner = 1;
+            for (int64_t d = dim + 1; d < rank; ++d) inner *= x.size(d);
+            put_ref(s_strided);
+            put(PyLong_FromLong(x.device().index()));
+            put(PyLong_FromLong(logn));
+            put(PyLong_FromLongLong(inner));
+            put(PyLong_FromLongLong(x.numel() / (len * inner)));
+            put(PyLong_FromLong(code));
+        } else {
+            put(PyLong_FromLong(x.device().index()));
+            put(PyLong_FromLong(logn));
+            put(PyLong_FromLongLong(x.numel() / len));
+            put(PyLong_FromLong(code));
+            put(PyBool_FromLong(ft));
+            put(PyBool_FromLong(err));
+            put_ref(a[3]);
+        }
+        put(PyBool_FromLong(inverse));
+        put_ref(a[5]);
+        PyObject* plan = PyDict_GetItemWithError(g_plans, key);  // borrowed
+        Py_DECREF(key);
+        if (!plan) {
+            if (PyErr_Occurred()) return nullptr;
+            Py_RETURN_NONE;
+        }
+        Py_INCREF(plan);
+        void* h = plan_handle(plan);
+        PyObject* r = nullptr;
+        if (h) {
+            r = execute(h, x, a[4]);
+        } else {
+            Py_INCREF(Py_None);
+            r = Py_None;
+        }
+        Py_DECREF(plan);
+        return r;
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
+// exec(plan, x, out): Plan.__call__, or None
+PyObject* fast_exec(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 3 || !g_exec || !ordinary(a[1]) || (a[2] != Py_None && !ordinary(a[2]))) Py_RETURN_NONE;
+    try {
+        const at::Tensor& x = THPVariable_Unpack(a[1]);
+        long long logn, batch, dtype, device;
+        if (!int_attr(a[0], s_logn, &logn) || !int_attr(a[0], s_batch, &batch) || !int_attr(a[0], s_dtype, &dtype) ||
+            !int_attr(a[0], s_device, &device))
+            Py_RETURN_NONE;
+        if (!x.is_cuda() || type_code(x) != dtype || x.numel() != (batch << logn) || x.device().index() != device || !x.is_contiguous())
+            Py_RETURN_NONE;
+        if (a[2] != Py_None) {
+            const at::Tensor& y = THPVariable_Unpack(a[2]);
+            if (!y.is_cuda() || !y.is_contiguous() || y.scalar_type() != x.scalar_type() || y.numel() != x.numel()) Py_RETURN_NONE;
+        }
+        void* h = plan_handle(a[0]);
+        if (!h) Py_RETURN_NONE;
+        return execute(h, x, a[2]);
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
+// ft_status(plan, launch): (detected, corrected, [located per block]) with one library call, or the negative status
+PyObject* ft_status(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 2 || !PyLong_Check(a[1])) {
+        PyErr_SetString(PyExc_TypeError, "ft_status(plan, launch)");
+        return nullptr;
+    }
+    void* h = plan_handle(a[0]);
+    const int launch = (int)PyLong_AsLong(a[1]);
+    int info[19] = {0}, nd = 0, nc = 0, nb = 0, rc = h ? g_info(h, info) : -1;
+    if (rc == 0) {
+        const int last = launch < 0 ? info[0] - 1 : launch;
+        std::vector<int> located(last < info[0] ? (size_t)info[1 + 6 * last + 3] : 0);  // the launch's grid
+        Py_BEGIN_ALLOW_THREADS
+        rc = g_status(h, &nd, &nc, launch, located.data(), (int)located.size(), &nb);
+        Py_END_ALLOW_THREADS
+        if (rc == 0) {
+            PyObject* list = PyList_New(nb);
+            if (!list) return nullptr;
+            for (int i = 0; i < nb; ++i) PyList_SET_ITEM(list, i, PyLong_FromLong(located[i]));
+            return Py_BuildValue("iiN", nd, nc, list);
+        }
+    }
+    return PyLong_FromLong(rc);
+}
+
+// bind(addresses of tfft_exec, tfft_ft_status and tfft_plan_info, plan dictionary)
+PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 4 || !PyDict_Check(a[3])) {
+        PyErr_SetString(PyExc_TypeError, "bind(exec, ft_status, plan_info, dict)");
+        return nullptr;
+    }
+    void* p[3];
+    for (int i = 0; i < 3; ++i) {
+        p[i] = PyLong_AsVoidPtr(a[i]);
+        if (!p[i] && PyErr_Occurred()) return nullptr;
+    }
+    Py_INCREF(a[3]);
+    Py_XDECREF(g_plans);
+    g_plans = a[3];
+    g_exec = (ExecFn)p[0];
+    g_status = (StatusFn)p[1];
+    g_info = (InfoFn)p[2];
+    Py_RETURN_NONE;
+}
+
+PyMethodDef kMethods[] = {
+    {"fft", (PyCFunction)(void (*)(void))fast_fft, METH_FASTCALL, nullptr},
+    {"exec", (PyCFunction)(void (*)(void))fast_exec, METH_FASTCALL, nullptr},
+    {"ft_status", (PyCFunction)(void (*)(void))ft_status, METH_FASTCALL, nullptr},
+    {"bind", (PyCFunction)(void (*)(void))bind, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_torch_binding", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__torch_binding(void) {
+    s_h = PyUnicode_InternFromString("_h");
+    s_value = PyUnicode_InternFromString("value");
+    s_logn = PyUnicode_InternFromString("logN");
+    s_batch = PyUnicode_InternFromString("batch");
+    s_dtype = PyUnicode_InternFromString("dtype");
+    s_device = PyUnicode_InternFromString("device");
+    s_strided = PyUnicode_InternFromString("strided");
+    return PyModule_Create(&kModule);
+}
