@@ -124,7 +124,7 @@ int tfft_exec_ws(tfft_plan plan, const void* in, void* out, void* workspace, voi
  * tfft_exec and copies the result back, then synchronises.  Replaces the
  * cudaMemcpy pair around the launches in initializeData()/test_turbofft()
  * (initializeData.h:39, main.cu:72).  Plans without FT whose batch spans at least
- * three chunks (64 MiB of whole signals, or one signal of up to 512 MiB) are pipelined: chunks of whole signals are copied in,
+ * three chunks (a sixteenth of the batch, 2 to 64 MiB of whole signals, or one signal of up to 512 MiB) are pipelined: chunks of whole signals are copied in,
  * transformed and copied out on three internal streams so both PCIe directions
  * overlap the kernels (use pinned host buffers).  Device staging buffers, the
  * three streams and their events are per device, grow-only, shared by all plans

@@ -51,7 +51,16 @@ std::map<int, StagePair> g_stage;
 // copy-in, transform and copy-out, and the events that order the slots.  Shared by all plans of the
 // device and kept until the library is unloaded, so that consecutive calls -- of one plan or of
 // several -- keep the pipeline full: the copy-out tail of one call overlaps the copy-in head of the next.
-constexpr size_t kPipeChunkBytes = 64u << 20;
+// A call fills and drains the pipeline once, during which only one PCIe direction is busy: about one chunk's copy at
+// either end.  So a call is cut into sixteen chunks (a sixteenth of its time is not overlapped), of at most 64 MiB (no
+// gain beyond, and six slots of that size are held) and at least 2 MiB (40 us of copying, which covers the dozen driver
+// calls that queue a chunk).  Bound: PCIe.  2^12 x 2^12 complex64 (128 MiB each way), which chunks of 64 MiB left
+// unpipelined: 4.84 -> 3.21 ms.
+constexpr size_t kPipeChunkMost = 64u << 20, kPipeChunkLeast = 2u << 20;
+size_t pipe_chunk_bytes(size_t call_bytes) {
+    const size_t want = call_bytes / 16;
+    return want < kPipeChunkLeast ? kPipeChunkLeast : (want > kPipeChunkMost ? kPipeChunkMost : want);
+}
 struct PipeSlots {
     void* in[3] = {nullptr, nullptr, nullptr};
     void* out[3] = {nullptr, nullptr, nullptr};
@@ -863,13 +872,13 @@ int tfft_exec_ws(tfft_plan p, const void* in, void* out, void* workspace, void* 
 }
 
 // Pipelined form of tfft_exec_host for plans without FT whose batch spans several chunks:
-// the batch is cut into chunks of whole signals (about 64 MiB); chunk i is copied in on one
+// the batch is cut into chunks of whole signals (pipe_chunk_bytes); chunk i is copied in on one
 // stream, transformed on a second and copied out on a third, three slots deep, so the two
 // PCIe directions and the kernels overlap.  Returns TFFT_ERR_UNSUPPORTED when the plan does
 // not qualify (the caller then takes the plain path).
 static int exec_host_pipelined(tfft_plan p, const void* in_host, void* out_host, cudaStream_t user, bool sync) {
     const size_t sig_bytes = ((size_t)1 << p->logn) * p->esize();
-    long long cb = (long long)(kPipeChunkBytes / sig_bytes);
+    long long cb = (long long)(pipe_chunk_bytes((size_t)p->batch * sig_bytes) / sig_bytes);
     // signals longer than a chunk travel one per chunk (up to 512 MiB each: six staging slots of that size)
     if (cb < 1 && sig_bytes <= ((size_t)512 << 20)) cb = 1;
     // chunk plans are ordinary launch plans over whole signals: strided-batch, single-pass and fused plans
