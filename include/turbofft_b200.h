@@ -151,6 +151,9 @@ size_t tfft_workspace_bytes(tfft_plan plan);
  * info must hold 1 + 3*6 ints. */
 int tfft_plan_info(tfft_plan plan, int* info);
 
+/* What the plan was created for; no device is touched. */
+int tfft_plan_shape(tfft_plan plan, int* logN, long long* batch, int* dtype, int* device);
+
 /* The three literals fft_codegen.py bakes into the generated source
  * (--err_inj, --err_smoothing, --err_threshold; fft_codegen.py:414,495,714-719)
  * as run-time values.  Defaults: 100, 1000, 1e-3. */

@@ -194,7 +194,7 @@ def _load_binding():
     _torch()  # the module's libtorch symbols
     from . import _torch_binding
 
-    entry = [C.cast(f, C.c_void_p).value for f in (lib().tfft_exec, lib().tfft_ft_status, lib().tfft_plan_info)]
+    entry = [C.cast(f, C.c_void_p).value for f in (lib().tfft_exec, lib().tfft_ft_status, lib().tfft_plan_info, lib().tfft_plan_shape)]
     _torch_binding.bind(*entry, _plan_cache)
     _binding = _torch_binding
     return _binding

@@ -36,6 +36,7 @@ SIGNATURES = {
     "tfft_host_sync": (C.c_int, [C.c_int]),
     "tfft_workspace_bytes": (C.c_size_t, [C.c_void_p]),
     "tfft_plan_info": (C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
+    "tfft_plan_shape": (C.c_int, [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_longlong), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "tfft_set_ft_params": (C.c_int, [C.c_void_p, C.c_double, C.c_double, C.c_double]),
     "tfft_set_correction": (C.c_int, [C.c_void_p, C.c_int]),
     "tfft_set_direction": (C.c_int, [C.c_void_p, C.c_int, C.c_double]),

@@ -95,7 +95,8 @@ struct DeviceGuard {
     bool ok = true;
     explicit DeviceGuard(int dev) {
         if (cudaGetDevice(&prev) != cudaSuccess) ok = false;
-        if (ok && prev != dev && cudaSetDevice(dev) != cudaSuccess) ok = false;
+        if (ok && prev == dev) prev = -1;  // nothing to put back
+        else if (ok && cudaSetDevice(dev) != cudaSuccess) ok = false;
     }
     ~DeviceGuard() {
         if (prev >= 0) cudaSetDevice(prev);
@@ -1054,6 +1055,15 @@ int tfft_plan_info(tfft_plan p, int* info) {
             for (int j = 0; j < 6; ++j) o[j] = 0;
         }
     }
+    return TFFT_OK;
+}
+
+int tfft_plan_shape(tfft_plan p, int* logN, long long* batch, int* dtype, int* device) {
+    if (!p || !logN || !batch || !dtype || !device) return TFFT_ERR_BAD_ARG;
+    *logN = p->logn;
+    *batch = p->batch;
+    *dtype = p->dtype;
+    *device = p->device;
     return TFFT_OK;
 }
 

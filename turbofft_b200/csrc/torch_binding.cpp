@@ -11,6 +11,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -22,12 +23,14 @@ namespace {
 typedef int (*ExecFn)(void*, const void*, void*, void*);
 typedef int (*StatusFn)(void*, int*, int*, int, int*, int, int*);
 typedef int (*InfoFn)(void*, int*);
+typedef int (*ShapeFn)(void*, int*, long long*, int*, int*);
 
 ExecFn g_exec = nullptr;
 StatusFn g_status = nullptr;
 InfoFn g_info = nullptr;
+ShapeFn g_shape = nullptr;
 PyObject* g_plans = nullptr;  // turbofft_b200._plan_cache
-PyObject *s_h, *s_value, *s_logn, *s_batch, *s_dtype, *s_device, *s_strided;
+PyObject *s_h, *s_value, *s_strided;
 
 // complex64 -> 0, complex128 -> 1 (the C ABI's dtype codes), anything else -> -1
 int type_code(const at::Tensor& x) {
@@ -36,22 +39,6 @@ int type_code(const at::Tensor& x) {
 }
 
 bool ordinary(PyObject* o) { return THPVariable_CheckExact(o); }
-
-// an int attribute of a Plan; false (no error set) if it is not one
-bool int_attr(PyObject* o, PyObject* name, long long* v) {
-    PyObject* a = PyObject_GetAttr(o, name);
-    if (!a) {
-        PyErr_Clear();
-        return false;
-    }
-    *v = PyLong_Check(a) ? PyLong_AsLongLong(a) : -1;
-    Py_DECREF(a);
-    if (PyErr_Occurred()) {
-        PyErr_Clear();
-        return false;
-    }
-    return true;
-}
 
 // the tfft_plan behind a Plan object, null for a destroyed one
 void* plan_handle(PyObject* plan) {
@@ -68,7 +55,7 @@ void* plan_handle(PyObject* plan) {
 // tensor's device.  None when the library reports an error: the Python path repeats the call and raises.
 PyObject* execute(void* plan, const at::Tensor& x, PyObject* out_obj) {
     at::Tensor y;
-    if (out_obj == Py_None) y = at::empty(x.sizes(), x.options());
+    if (out_obj == Py_None) y = at::detail::empty_cuda(x.sizes(), x.scalar_type(), x.device(), c10::nullopt);
     else y = THPVariable_Unpack(out_obj);
     void* stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
     int rc;
@@ -83,6 +70,35 @@ PyObject* execute(void* plan, const at::Tensor& x, PyObject* out_obj) {
         return out_obj;
     }
     return THPVariable_Wrap(std::move(y));
+}
+
+struct KeyFields {
+    int64_t device, logn, batch, inner, thread_bs;  // inner: 0 for the last axis
+    double expo;
+    int64_t flags;
+    bool operator==(const KeyFields& o) const {
+        return device == o.device && logn == o.logn && batch == o.batch && inner == o.inner && thread_bs == o.thread_bs &&
+               expo == o.expo && flags == o.flags;
+    }
+};
+struct KeySlot {
+    KeyFields fields;
+    PyObject* key;
+};
+constexpr int kKeySlots = 64;
+KeySlot g_keys[kKeySlots];  // under the interpreter lock
+
+// The key turbofft_b200.fft files this call's plan under, kept in `slot`
+PyObject* make_key(PyObject* const* a, const KeyFields& f, int64_t outer, int code, int ft, int err, int inverse, KeySlot& slot) {
+    PyObject* key = f.inner ? Py_BuildValue("(OLLLLiOO)", s_strided, (long long)f.device, (long long)f.logn, (long long)f.inner,
+                                            (long long)outer, code, inverse ? Py_True : Py_False, a[5])
+                            : Py_BuildValue("(LLLiOOOOO)", (long long)f.device, (long long)f.logn, (long long)f.batch, code,
+                                            ft ? Py_True : Py_False, err ? Py_True : Py_False, a[3], inverse ? Py_True : Py_False, a[5]);
+    if (!key) return nullptr;
+    Py_XDECREF(slot.key);
+    slot.fields = f;
+    slot.key = key;
+    return key;
 }
 
 // fft(x, ft, err, thread_bs, out, norm_exponent, inverse, dim): the transform along one axis, or None
@@ -105,39 +121,24 @@ PyObject* fast_fft(PyObject*, PyObject* const* a, Py_ssize_t n) {
         }
         const int ft = PyObject_IsTrue(a[1]), err = PyObject_IsTrue(a[2]), inverse = PyObject_IsTrue(a[6]);
         if (ft < 0 || err < 0 || inverse < 0) return nullptr;
-        // the keys turbofft_b200.fft files its plans under
         const bool strided = dim != rank - 1;
         if (strided && (ft || err || a[4] != Py_None)) Py_RETURN_NONE;
-        PyObject* key = PyTuple_New(strided ? 8 : 9);
-        if (!key) return nullptr;
-        int k = 0;
-        auto put = [&](PyObject* o) { PyTuple_SET_ITEM(key, k++, o); };
-        auto put_ref = [&](PyObject* o) {
-            Py_INCREF(o);
-            put(o);
-        };
-        if (strided) {
-            int64_t inner = 1;
-            for (int64_t d = dim + 1; d < rank; ++d) inner *= x.size(d);
-            put_ref(s_strided);
-            put(PyLong_FromLong(x.device().index()));
-            put(PyLong_FromLong(logn));
-            put(PyLong_FromLongLong(inner));
-            put(PyLong_FromLongLong(x.numel() / (len * inner)));
-            put(PyLong_FromLong(code));
-        } else {
-            put(PyLong_FromLong(x.device().index()));
-            put(PyLong_FromLong(logn));
-            put(PyLong_FromLongLong(x.numel() / len));
-            put(PyLong_FromLong(code));
-            put(PyBool_FromLong(ft));
-            put(PyBool_FromLong(err));
-            put_ref(a[3]);
+        int64_t inner = 1;
+        for (int64_t d = dim + 1; d < rank; ++d) inner *= x.size(d);
+        // a program repeats a handful of shapes: their key tuples are kept, the plans stay the dictionary's
+        const int64_t thread_bs = PyLong_Check(a[3]) ? PyLong_AsLongLong(a[3]) : -1;
+        const double expo = PyFloat_Check(a[5]) ? PyFloat_AS_DOUBLE(a[5]) : 2.0;
+        if (thread_bs < 0 || expo > 1.0) {
+            PyErr_Clear();
+            Py_RETURN_NONE;
         }
-        put(PyBool_FromLong(inverse));
-        put_ref(a[5]);
+        const KeyFields fields = {x.device().index(), logn, x.numel() / len, strided ? inner : 0, thread_bs, expo,
+                                  code | ft << 1 | err << 2 | inverse << 3};
+        KeySlot& slot = g_keys[(fields.batch * 31 + fields.logn * 7 + fields.flags) & (kKeySlots - 1)];
+        PyObject* key = slot.key && slot.fields == fields ? slot.key : nullptr;
+        if (!key) key = make_key(a, fields, x.numel() / (len * inner), code, ft, err, inverse, slot);
+        if (!key) return nullptr;
         PyObject* plan = PyDict_GetItemWithError(g_plans, key);  // borrowed
-        Py_DECREF(key);
         if (!plan) {
             if (PyErr_Occurred()) return nullptr;
             Py_RETURN_NONE;
@@ -164,18 +165,16 @@ PyObject* fast_exec(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (n != 3 || !g_exec || !ordinary(a[1]) || (a[2] != Py_None && !ordinary(a[2]))) Py_RETURN_NONE;
     try {
         const at::Tensor& x = THPVariable_Unpack(a[1]);
-        long long logn, batch, dtype, device;
-        if (!int_attr(a[0], s_logn, &logn) || !int_attr(a[0], s_batch, &batch) || !int_attr(a[0], s_dtype, &dtype) ||
-            !int_attr(a[0], s_device, &device))
-            Py_RETURN_NONE;
+        void* h = plan_handle(a[0]);
+        int logn, dtype, device;
+        long long batch;
+        if (!h || g_shape(h, &logn, &batch, &dtype, &device) != 0) Py_RETURN_NONE;
         if (!x.is_cuda() || type_code(x) != dtype || x.numel() != (batch << logn) || x.device().index() != device || !x.is_contiguous())
             Py_RETURN_NONE;
         if (a[2] != Py_None) {
             const at::Tensor& y = THPVariable_Unpack(a[2]);
             if (!y.is_cuda() || !y.is_contiguous() || y.scalar_type() != x.scalar_type() || y.numel() != x.numel()) Py_RETURN_NONE;
         }
-        void* h = plan_handle(a[0]);
-        if (!h) Py_RETURN_NONE;
         return execute(h, x, a[2]);
     } catch (const std::exception& e) {
         PyErr_SetString(PyExc_RuntimeError, e.what());
@@ -208,23 +207,24 @@ PyObject* ft_status(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return PyLong_FromLong(rc);
 }
 
-// bind(addresses of tfft_exec, tfft_ft_status and tfft_plan_info, plan dictionary)
+// bind(addresses of tfft_exec, tfft_ft_status, tfft_plan_info and tfft_plan_shape, plan dictionary)
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (n != 4 || !PyDict_Check(a[3])) {
-        PyErr_SetString(PyExc_TypeError, "bind(exec, ft_status, plan_info, dict)");
+    if (n != 5 || !PyDict_Check(a[4])) {
+        PyErr_SetString(PyExc_TypeError, "bind(exec, ft_status, plan_info, plan_shape, dict)");
         return nullptr;
     }
-    void* p[3];
-    for (int i = 0; i < 3; ++i) {
+    void* p[4];
+    for (int i = 0; i < 4; ++i) {
         p[i] = PyLong_AsVoidPtr(a[i]);
         if (!p[i] && PyErr_Occurred()) return nullptr;
     }
-    Py_INCREF(a[3]);
+    Py_INCREF(a[4]);
     Py_XDECREF(g_plans);
-    g_plans = a[3];
+    g_plans = a[4];
     g_exec = (ExecFn)p[0];
     g_status = (StatusFn)p[1];
     g_info = (InfoFn)p[2];
+    g_shape = (ShapeFn)p[3];
     Py_RETURN_NONE;
 }
 
@@ -242,10 +242,6 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_torch_binding", nullptr, -1, kMe
 PyMODINIT_FUNC PyInit__torch_binding(void) {
     s_h = PyUnicode_InternFromString("_h");
     s_value = PyUnicode_InternFromString("value");
-    s_logn = PyUnicode_InternFromString("logN");
-    s_batch = PyUnicode_InternFromString("batch");
-    s_dtype = PyUnicode_InternFromString("dtype");
-    s_device = PyUnicode_InternFromString("device");
     s_strided = PyUnicode_InternFromString("strided");
     return PyModule_Create(&kModule);
 }
