@@ -45,6 +45,22 @@ def collect_instances(rows):
     return seen
 
 
+def narrow_instances(rows, datatype):
+    """The multi-launch kernels of the rows again with fewer lines per tile, down to runs of 32 bytes: what
+    the planner picks for batches whose tiles would leave SMs without a block (capi.cu, adjust_tiles).
+    From 2^22 points on a single signal has tiles enough."""
+    least = 2 if datatype == "float2" else 1
+    out = []
+    for logn in sorted(rows):
+        if rows[logn].launches < 2 or logn >= 22:
+            continue
+        for l in launches_of_row(rows[logn]):
+            for logc in range(l.logc - 1, least - 1, -1):
+                if (1 << (l.logm - l.loge + logc)) >= 32:
+                    out.append((l.logm, l.loge, logc, l.role))
+    return out
+
+
 def write_if_changed(path, text):
     os.makedirs(os.path.dirname(path), exist_ok=True)
     if os.path.exists(path) and open(path).read() == text:
@@ -87,13 +103,14 @@ def main(argv=None):
 
     if mode == 0:
         # strided-line kernels of every length 2^1..2^12 for the strided-batch plan
-        # (tfft_plan_create_strided), whatever lengths the launch rows above happen to use
-        for key in STRIDED_LINES[args.datatype]:
+        # (tfft_plan_create_strided), whatever lengths the launch rows above happen to use, and narrower
+        # tiles of the rows' own kernels
+        for key in STRIDED_LINES[args.datatype] + narrow_instances(rows, args.datatype):
             if key not in inst:
                 inst.append(key)
     if mode == 3:
-        # checksum-based correction exists for single and last launches with at least one exchange
-        inst = [(logm, loge, logc, role) for (logm, loge, logc, role) in inst if role != 1 and logm > loge]
+        # checksum-based correction exists for single and last launches of 32 points and more
+        inst = [(logm, loge, logc, role) for (logm, loge, logc, role) in inst if role != 1 and logm >= 5]
     ctype = "float" if args.datatype == "float2" else "double"
     dt = 0 if args.datatype == "float2" else 1
     odir = os.path.join(args.out, args.datatype)

@@ -150,6 +150,9 @@ template <> __device__ __forceinline__ float2 acc_zero<float2>() { return make_f
 // 2^16 x 1 10.9 -> 6.0 us, 2^22 x 1 41 -> 34 us, 2^16 x 512 175 -> 170 us (complex64).  The start signal stands before
 // the stores because a launch placed earlier finds the SMs still occupied and is spread unevenly: with the signal at
 // the top of the kernel 2^16 x 8 takes 9.6 us, here 7.1 us.
+// Not for lines of 2 and 4 points, whose launches are hundreds of thousands of blocks of a few KB: there the two
+// instructions cost each block more than the launch gains (2^2 complex64, 1 GiB: 542 us with them, 327 without).
+__host__ __device__ constexpr bool dependent_launch(int logm) { return logm > 2; }
 __device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;"); }
 
@@ -283,6 +286,8 @@ struct Cfg {
     // One thread per line (M == E, whole signals): lines are too short to be read coalesced
     // by their owner, so the tile -- contiguous in memory -- is staged through shared memory:
     // cooperative coalesced copy in, each thread picks up its line (pitch M + 1), and back.
+    // Bound: HBM.  32-point complex64 lines in one thread each (1 GiB): 369 us as four threads of 8 points, whose loads
+    // touch a 128-byte line per 32 bytes (343 us with those staged as well), 311 us in this form.
     static constexpr bool STAGED_IO = (ROLE == ROLE_SINGLE && S == 1 && TPL == 1 && LOGM >= 2);
     static constexpr int SMEM_ELEMS = STAGED_IO ? (M + 1) * C : (S > 1 ? (LAYOUT_COLS ? MPAD * C : PITCH * C) : 0);
     static constexpr size_t SMEM_BYTES = (size_t)SMEM_ELEMS * 2 * sizeof(T);
@@ -500,8 +505,8 @@ struct Fft {
                 y[i].y *= a.scale_y;
             }
         }
-        let_next_launch_start();
-        if constexpr (K::STAGED_IO) {
+        if constexpr (dependent_launch(LOGM)) let_next_launch_start();
+        if constexpr (K::STAGED_IO && CS != 2) {
             // every thread only touches its own line here, so no barrier is needed before
 #pragma unroll
             for (int i = 0; i < E; ++i) sm[c * (K::M + 1) + i] = y[i];
@@ -611,7 +616,7 @@ struct Fft {
     template <bool DO_FT, bool DO_INJ, int CS = 0, bool L2ONLY = false, typename Hook = NoHook>
     static __device__ __forceinline__ void tile(const KernelArgs<T>& a, C* sm, long long tile_id, bool inject,
                                                 const FtRegs& f, A& tin, A& tout, Hook after_loads = Hook()) {
-        static_assert(CS == 0 || (!K::STAGED_IO && ROLE != ROLE_FIRST), "checksum correction: single and last launches only");
+        static_assert(CS == 0 || ROLE != ROLE_FIRST, "checksum correction: single and last launches only");
         const Geom g = decode(a, tile_id);
         int s, c;
         map_thread<K::CFAST_IN>(s, c);
@@ -800,7 +805,7 @@ __global__ void __launch_bounds__((Cfg<T, LOGM, LOGE, LOGC, ROLE>::THREADS),
 fft_kernel(const __grid_constant__ KernelArgs<T> a) {
     extern __shared__ __align__(16) unsigned char tfft_smem_raw[];
     typedef typename Cplx<T>::type C;
-    wait_for_previous_launch();
+    if constexpr (dependent_launch(LOGM)) wait_for_previous_launch();
     Fft<T, LOGM, LOGE, LOGC, ROLE, FT>::run(a, reinterpret_cast<C*>(tfft_smem_raw));
 }
 
