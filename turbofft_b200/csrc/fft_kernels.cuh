@@ -141,6 +141,18 @@ __device__ __forceinline__ float acc_sum(float2 acc) { return acc.x + acc.y; }
 template <> __device__ __forceinline__ float2 acc_zero<float2>() { return make_float2(0.0f, 0.0f); }
 #endif
 
+// A result leaves the SM without taking a line of L1: what a block reads again (stage twiddles, checksum weights) stays
+// there instead.  Bound: L1 of the launches with 1024-point lines, whose 32- and 64-byte runs take a line each, and of the
+// FT kernels, which read their weights for every tile.  Before -> after (complex64, sustained): 2^20 x 256 1638 -> 1610 us,
+// 2^21 x 128 1817 -> 1766, 2^20 x 256 with detection 1786 -> 1752, with correction 1805 -> 1770, 2^12 x 2^14 with
+// detection 209.3 -> 206.9; lines of 256 and 512 points do not change.
+__device__ __forceinline__ void store_result(float2* p, float2 v) {
+    asm volatile("st.global.L1::no_allocate.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void store_result(double2* p, double2 v) {
+    asm volatile("st.global.L1::no_allocate.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v.x), "d"(v.y) : "memory");
+}
+
 // Programmatic dependent launch.  No block touches global data before the launch before it has completed and its
 // stores are visible (wait_for_previous_launch); once every block has got as far as the stores of its first tile, the
 // next launch of the stream may place its blocks in the slots that this one's tail leaves empty (let_next_launch_start).
@@ -525,7 +537,7 @@ struct Fft {
             for (int i = 0; i < E; ++i) {
                 if (!in_range(a, o0 + (long long)i * TPL * g.out_rs, 4)) continue;
                 if (CS == 2) dst[(long long)i * TPL * g.out_rs] = csub(dst[(long long)i * TPL * g.out_rs], y[i]);
-                else dst[(long long)i * TPL * g.out_rs] = y[i];
+                else store_result(dst + (long long)i * TPL * g.out_rs, y[i]);
             }
         }
     }
