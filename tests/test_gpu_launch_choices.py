@@ -1,0 +1,150 @@
+"""The choices that a plan makes by batch: narrower tiles for few signals, one thread per 32-point line, launches that
+overlap the drain of the one before, host calls cut in chunks; and the native call path against the general one."""
+import numpy as np
+import pytest
+
+from oracle import fft_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+CD = {0: np.complex64, 1: np.complex128}
+
+
+def _same(torch, a, b):
+    return torch.equal(torch.view_as_real(a), torch.view_as_real(b))
+
+
+# smallest and largest two-launch sizes, a three-launch size (complex128 2^20), batches around the 128 and 512 tile limits
+@pytest.mark.parametrize("dtype,logn", [(0, 15), (0, 16), (0, 18), (0, 20), (0, 21), (1, 13), (1, 16), (1, 17), (1, 20)])
+@pytest.mark.parametrize("batch", [1, 2, 5, 16, 33])
+def test_narrow_tiles_give_the_bits_of_wide_ones(torch_cuda, dtype, logn, batch):
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    if batch << logn > 1 << 22:
+        batch = max(1, (1 << 22) >> logn) + 1  # largest batch worth its time, odd
+    x = torch.from_numpy(orc.make_input(batch, 1 << logn, CD[dtype], seed=logn + batch)).cuda()
+    y = tf.Plan(logn, batch, dtype)(x)
+    wide = max(batch, min(600, (1 << 25) >> logn))  # enough tiles for the row's own tiles in every launch
+    xw = torch.zeros(wide, 1 << logn, dtype=x.dtype, device="cuda")
+    xw[:batch] = x
+    yw = tf.Plan(logn, wide, dtype)(xw)
+    assert _same(torch, y, yw[:batch])
+    assert orc.rel_l2(y[-1:].cpu().numpy(), orc.fft_forward(x[-1:].cpu().numpy())) <= orc.tolerance(CD[dtype], logn)
+
+
+@pytest.mark.parametrize("if_ft", [0, 1])
+@pytest.mark.parametrize("batch", [1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 4097])
+def test_32_point_lines_at_the_edges_of_a_tile(torch_cuda, batch, if_ft):
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    x_np = orc.make_input(batch, 32, np.complex64, seed=batch)
+    x = torch.from_numpy(x_np).cuda()
+    guard = torch.full((batch + 2, 32), 7 + 7j, dtype=torch.complex64, device="cuda")
+    plan = tf.Plan(5, batch, 0, if_ft=if_ft, thread_bs=2)
+    plan(x, guard[1:-1])
+    assert orc.rel_l2(guard[1:-1].cpu().numpy(), orc.fft_forward(x_np)) <= orc.tolerance(np.complex64, 5)
+    assert bool((guard[[0, -1]] == 7 + 7j).all())  # nothing stored beside the batch
+    if if_ft:
+        assert plan.ft_status()[0] == 0
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("logn,batch", [(2, 5000), (5, 700), (12, 3), (16, 2), (16, 600), (22, 1)])
+def test_a_chain_of_launches_reads_what_the_one_before_wrote(torch_cuda, logn, batch, dtype):
+    """Forward and back, in place and out of place, twenty times without a wait in between."""
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    x = torch.from_numpy(orc.make_input(batch, 1 << logn, CD[dtype], seed=3)).cuda()
+    fwd, bwd = tf.Plan(logn, batch, dtype), tf.Plan(logn, batch, dtype)
+    bwd.set_direction(True, 1.0 / (1 << logn))
+    y, z = x.clone(), torch.empty_like(x)
+    for _ in range(10):
+        fwd(y, z)
+        bwd(z, z)
+        y.copy_(z)  # a launch of another library between two of ours
+    z = y
+    for _ in range(10):
+        a = fwd(z)
+        z = bwd(a)
+        del a       # its memory is free for the next call's output
+    # forty transforms, each within the tolerance of one
+    assert float(torch.linalg.vector_norm(z - x) / torch.linalg.vector_norm(x)) <= 40 * orc.tolerance(CD[dtype], logn)
+    # the same steps with a wait after each give the same bits
+    y = x.clone()
+    for _ in range(20):
+        y = fwd(y)
+        torch.cuda.synchronize()
+        y = bwd(y)
+        torch.cuda.synchronize()
+    assert _same(torch, y, z)
+
+
+# 2 MiB chunks: just under and over three of them, a ragged last one, and a call of more than sixteen
+@pytest.mark.parametrize("logn,batch", [(10, 767), (10, 768), (10, 769), (12, 1000), (12, 4099), (18, 5)])
+def test_host_calls_of_a_few_chunks(torch_cuda, logn, batch):
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    x = torch.from_numpy(orc.make_input(batch, 1 << logn, np.complex64, seed=9)).pin_memory()
+    plan = tf.Plan(logn, batch, 0)
+    for _ in range(2):
+        assert _same(torch, plan.exec_host(x), plan(x.cuda()).cpu())
+
+
+def test_native_call_path_and_general_one_agree(torch_cuda):
+    """Calls that the native path takes, and near ones that it leaves to the general path."""
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+
+    class Sub(torch.Tensor):
+        pass
+
+    x = torch.from_numpy(orc.make_input(12, 256, np.complex64, seed=1)).cuda()
+    want = torch.fft.fft(x.to(torch.complex128))
+
+    def close(y, w):
+        return float(torch.linalg.vector_norm(y.as_subclass(torch.Tensor) - w) / torch.linalg.vector_norm(w)) <= orc.tolerance(np.complex64, 8)
+
+    for _ in range(2):  # the first call makes the plan, the second finds it
+        assert close(tf.fft(x), want) and close(tf.fft(x.as_subclass(Sub)), want)
+        assert close(tf.fft(x.view(3, 4, 256)), want.view(3, 4, 256))
+        assert close(tf.fft(x.t().contiguous().t()), want)           # strided view: copied first
+        assert close(tf.fft(x.view(3, 4, 256), dim=1), torch.fft.fft(x.view(3, 4, 256).to(torch.complex128), dim=1))
+        assert close(tf.fft(x[0]), want[0]) and close(tf.ifft(tf.fft(x)), x)
+        out = torch.empty_like(x)
+        assert close(tf.fft(x, out=out), want) and close(out, want)
+        odd = torch.empty(12 * 256 + 1, dtype=torch.complex64, device="cuda")[1:].view(12, 256)  # 8 bytes off a 16-byte boundary
+        odd.copy_(x)
+        assert close(tf.fft(odd), want)
+        for norm in ("ortho", "forward"):
+            assert close(tf.fft(x, norm=norm), torch.fft.fft(x.to(torch.complex128), norm=norm))
+    for bad in (x[:, :255].contiguous(), x.cpu(), x.real.contiguous()):
+        with pytest.raises(Exception):
+            tf.fft(bad)
+    plan = tf.Plan(8, 12, 0)
+    for args in ((x[:11].contiguous(),), (x.to(torch.complex128),), (x.cpu(),), (x, torch.empty(3, 256, dtype=x.dtype, device="cuda"))):
+        with pytest.raises(ValueError):
+            plan(*args)
+    assert close(plan(x), want)
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_status_counts_come_from_the_last_exec(torch_cuda, dtype):
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    x = torch.from_numpy(orc.make_input(96, 4096, CD[dtype], seed=2)).cuda()
+    plan = tf.Plan(12, 96, dtype, if_ft=1, if_err=1, thread_bs=4)
+    assert plan.ft_status()[:2] == (0, 0)          # before the first exec
+    plan.set_ft_params(1e5, 1000.0, 1e-3)
+    for _ in range(3):
+        plan(x)
+        nd, nc, located = plan.ft_status()
+        assert nd == nc == sum(k != -1 for k in located) == len(located) > 0
+    plan.set_injection(False)
+    plan(x)
+    assert plan.ft_status()[:2] == (0, 0)
