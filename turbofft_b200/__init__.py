@@ -34,6 +34,15 @@ def _dtype_code(t) -> int:
     raise TypeError(f"turbofft_b200 supports complex64 and complex128, got {t}")
 
 
+def _plain(x):
+    """Contiguous, with torch's lazy conjugate and negative bits applied: the kernels read the memory as it lies."""
+    return x.resolve_conj().resolve_neg().contiguous()
+
+
+def _lazy(x) -> bool:
+    return x.is_conj() or x.is_neg()
+
+
 class Plan:
     """One (logN, batch, dtype, FT mode) plan on one device."""
 
@@ -93,10 +102,10 @@ class Plan:
             raise ValueError("tensor does not match the plan")
         if x.device.index != self.device:
             raise ValueError("tensor is on another device than the plan")
-        x = x.contiguous()
+        x = _plain(x)
         if out is None:
             out = torch.empty_like(x)
-        elif not (out.is_cuda and out.is_contiguous() and out.dtype == x.dtype and out.numel() == x.numel()):
+        elif not (out.is_cuda and out.is_contiguous() and out.dtype == x.dtype and out.numel() == x.numel()) or _lazy(out):
             raise ValueError("bad output tensor")
         stream = torch.cuda.current_stream(x.device).cuda_stream
         self.exec_ptr(x.data_ptr(), out.data_ptr(), stream)
@@ -107,7 +116,9 @@ class Plan:
         torch = _torch()
         if x.is_cuda or _dtype_code(x.dtype) != self.dtype or x.numel() != self.batch << self.logN:
             raise ValueError("tensor does not match the plan")
-        x = x.contiguous()
+        x = _plain(x)
+        if out is not None and _lazy(out):
+            raise ValueError("bad output tensor")
         if out is None:
             out = torch.empty_like(x, pin_memory=x.is_pinned())
         self.exec_host_ptr(x.data_ptr(), out.data_ptr(), torch.cuda.current_stream(self.device).cuda_stream)
@@ -119,7 +130,8 @@ class Plan:
         turbofft_b200.host_sync(device) has returned."""
         torch = _torch()
         if x.is_cuda or out.is_cuda or _dtype_code(x.dtype) != self.dtype or x.numel() != self.batch << self.logN \
-                or out.dtype != x.dtype or out.numel() != x.numel() or not (x.is_contiguous() and out.is_contiguous()):
+                or out.dtype != x.dtype or out.numel() != x.numel() or not (x.is_contiguous() and out.is_contiguous()) \
+                or _lazy(x) or _lazy(out):
             raise ValueError("tensors do not match the plan")
         self.exec_host_async_ptr(x.data_ptr(), out.data_ptr(), torch.cuda.current_stream(self.device).cuda_stream)
         return out
@@ -206,7 +218,7 @@ _NORM_FWD = {None: 0.0, "backward": 0.0, "ortho": -0.5, "forward": -1.0}  # expo
 def _fft_strided(x, dim: int, norm, inverse: bool):
     """Transform along a middle axis of a contiguous tensor: [outer][N][inner], lines strided by inner."""
     torch = _torch()
-    x = x.contiguous()
+    x = _plain(x)
     n = x.shape[dim]
     logn = n.bit_length() - 1
     inner = 1

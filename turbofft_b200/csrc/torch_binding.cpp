@@ -5,7 +5,7 @@
 // (attribute reads, a key tuple, reshape, ctypes argument conversion) kept the caller busy for 15.
 // Here a call reads the tensor's fields through ATen, looks the plan up in the SAME dictionary the
 // Python side keeps, allocates the output and calls tfft_exec.  Whatever is not an ordinary call --
-// a plan that does not exist yet, a tensor that is not on a GPU, not contiguous, of
+// a plan that does not exist yet, a tensor that is not on a GPU, not contiguous, lazily conjugated, of
 // another type or length -- returns None, and the Python code does what it always did, errors included.
 // The module links nothing of the library: it is handed the address of the tfft_exec that _lib.py loaded.
 #include <Python.h>
@@ -38,7 +38,13 @@ int type_code(const at::Tensor& x) {
     return t == at::kComplexFloat ? 0 : (t == at::kComplexDouble ? 1 : -1);
 }
 
-bool ordinary(PyObject* o) { return THPVariable_CheckExact(o); }
+// A plain torch.Tensor whose memory is its value: no subclass, no lazy conjugate or negative bit (x.conj() is a
+// contiguous view of x's memory; the Python path applies the bit first)
+bool ordinary(PyObject* o) {
+    if (!THPVariable_CheckExact(o)) return false;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    return !t.is_conj() && !t.is_neg();
+}
 
 // the tfft_plan behind a Plan object, null for a destroyed one
 void* plan_handle(PyObject* plan) {

@@ -86,6 +86,7 @@ class DeviceBackend:
         return out
 
     def permute102(self, x, a: int, b: int, run: int):
+        x = x.resolve_conj().resolve_neg()  # the caller's signal comes in here
         out = self.torch.empty_like(x)
         _lib.check(lib().tfft_permute102(x.data_ptr(), out.data_ptr(), a, b, run, self.dt, self._stream()), "tfft_permute102")
         return out
@@ -398,7 +399,7 @@ class FusedFourStepFFT(FourStepFFT):
     def __call__(self, x_local):
         P, r = self.world, self.rank
         n1, n2, n1l, n2l = self.n1, self.n2, self.n1 // P, self.n2 // P
-        x_local = x_local.contiguous()
+        x_local = x_local.resolve_conj().resolve_neg().contiguous()
         if self.G > 1:
             if self.exchange == "dma":
                 tmp = self._exchange_dma(x_local, 0, n1l, n2, n1, r * n1l, False, self.l1, self.torch.empty_like(x_local))
@@ -474,6 +475,7 @@ class SingleProcessFourStep:
         import torch
 
         P = len(self.devices)
+        x_parts = [x.resolve_conj().resolve_neg() for x in x_parts]
         outs = [torch.empty_like(x) for x in x_parts]
         for x in x_parts:                      # inputs were produced on torch's streams
             torch.cuda.synchronize(x.device)
