@@ -114,11 +114,21 @@ int tfft_exec(tfft_plan plan, const void* in, void* out, void* stream);
  * intermediate result of multi-launch plans in a buffer the plan owns, which two overlapping
  * execs would share).  workspace: tfft_scratch_bytes(plan) bytes of device memory, 256-byte
  * aligned, private to this exec until it has completed (NULL when that is 0: one-launch and
- * single-pass plans).  Plans without FT only (the FT status buffers are per plan), and not
+ * single-pass plans).  Plans without FT only (the FT status buffers are per plan) unless the plan comes
+ * from tfft_plan_create_ws, and not
  * fused plans (tfft_plan_fuse_launches): TFFT_ERR_UNSUPPORTED otherwise.  The reference's launcher is single-threaded and
  * synchronises after every launch (main.cu:58); it has nothing to share. */
 size_t tfft_scratch_bytes(tfft_plan plan);
 int tfft_exec_ws(tfft_plan plan, const void* in, void* out, void* workspace, void* stream);
+
+/* tfft_plan_create without scratch buffers, for a plan that many callers share (turbofft_b200.fft
+ * keeps one per shape): it runs through tfft_exec_ws only, FT modes included, and execs on any
+ * streams and from any host threads may overlap.  tfft_scratch_bytes counts the second buffer that
+ * correcting 3-launch plans need.  With FT, tfft_ft_status reports whichever exec wrote last and
+ * does not wait for it.  tfft_exec of a multi-launch plan of this kind, tfft_exec_host and
+ * tfft_plan_fuse_launches return TFFT_ERR_UNSUPPORTED.  The reference has no counterpart. */
+int tfft_plan_create_ws(tfft_plan* plan, int logN, long long batch, int dtype, int if_ft, int if_err,
+                        int thread_bs, const char* param_csv, int device);
 
 /* Same transform with HOST buffers: copies batch*N elements to the device, runs
  * tfft_exec and copies the result back, then synchronises.  Replaces the

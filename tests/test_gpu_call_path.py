@@ -49,3 +49,99 @@ def test_lazy_conjugate_and_negative_bits_are_applied(torch_cuda, dtype, lazy):
     got, want = two(list(view.reshape(2, -1))), two(list(value.reshape(2, -1)))
     assert all(_same(torch, a, b) for a, b in zip(got, want))
     two.close()
+
+
+# two launches, three launches (complex128 2^20), with and without FT; kernels long enough to overlap
+SHARED = [(0, 16, 64, False, False), (1, 17, 32, False, False), (0, 22, 4, False, False), (0, 18, 32, True, False),
+          (1, 20, 4, True, True)]
+
+
+def _shared_plans(tf, logn):
+    return [p for k, p in tf._plan_cache.items() if k[0] != "strided" and k[1] == logn]
+
+
+@pytest.mark.parametrize("dtype,logn,batch,ft,err", SHARED)
+def test_calls_of_one_shape_share_nothing(torch_cuda, dtype, logn, batch, ft, err):
+    """Calls of one shape on several streams and from several threads overlap; the cached plan they share has no
+    buffer of its own that they could overwrite for each other."""
+    import threading
+
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    xs = [torch.from_numpy(orc.make_input(batch, 1 << logn, CD[dtype], seed=s)).cuda() for s in range(3)]
+    call = lambda x: tf.fft(x, ft=ft, err=err)  # noqa: E731
+    call(xs[0])
+    size = (batch << logn) * (8 << dtype)
+    assert all(p.workspace_bytes < size for p in _shared_plans(tf, logn))
+    want = []
+    for x in xs:
+        want.append(call(x))
+        torch.cuda.synchronize()
+    # one thread, a stream per input
+    streams = [torch.cuda.Stream() for _ in xs]
+    got = [[] for _ in xs]
+    for _ in range(6):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(call(xs[i]))
+    torch.cuda.synchronize()
+    assert all(_same(torch, y, want[i]) for i in range(3) for y in got[i])
+    # a thread per input, all on one stream and then each on its own
+    for own_stream in (False, True):
+        got = [[] for _ in xs]
+
+        def work(i):
+            with torch.cuda.stream(streams[i if own_stream else 0]):
+                for _ in range(10):
+                    got[i].append(call(xs[i]))
+
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+        [t.start() for t in threads]
+        [t.join() for t in threads]
+        torch.cuda.synchronize()
+        assert all(len(got[i]) == 10 and all(_same(torch, y, want[i]) for y in got[i]) for i in range(3))
+
+
+@pytest.mark.parametrize("dtype,logn,batch,ft,err", SHARED)
+def test_captured_calls_beside_ordinary_ones(torch_cuda, dtype, logn, batch, ft, err):
+    """A captured call keeps its intermediate buffer in the graph's own pool: it can be replayed while the same shape
+    runs on another stream."""
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    x, z = (torch.from_numpy(orc.make_input(batch, 1 << logn, CD[dtype], seed=s)).cuda() for s in (7, 8))
+    want_x, want_z = tf.fft(x, ft=ft, err=err), tf.fft(z, ft=ft, err=err)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = tf.fft(x, ft=ft, err=err)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    got = []
+    for _ in range(5):
+        graph.replay()
+        with torch.cuda.stream(side):
+            got.append(tf.fft(z, ft=ft, err=err))
+    torch.cuda.synchronize()
+    assert _same(torch, y, want_x) and all(_same(torch, g, want_z) for g in got)
+
+
+def test_plans_without_scratch_refuse_what_needs_it(torch_cuda):
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    lib = tf.lib()
+    x = torch.from_numpy(orc.make_input(2, 1 << 16, np.complex64, seed=1)).cuda()
+    y = torch.empty_like(x)
+    plan = tf.Plan(16, 2, 0, own_scratch=False)
+    assert lib.tfft_exec(plan._h, x.data_ptr(), y.data_ptr(), 0) == -2
+    assert lib.tfft_exec_ws(plan._h, x.data_ptr(), y.data_ptr(), None, 0) == -1
+    assert lib.tfft_exec_host(plan._h, x.data_ptr(), y.data_ptr(), 0) == -2
+    assert lib.tfft_plan_fuse_launches(plan._h, 2, 1) == -2
+    assert _same(torch, plan(x), tf.Plan(16, 2, 0)(x))
+    # the second buffer of three launches that repair by recomputing
+    both = [tf.Plan(22, 1, 0, if_ft=1, if_err=1, own_scratch=own) for own in (True, False)]
+    assert [lib.tfft_scratch_bytes(p._h) for p in both] == [1 << 25, 2 << 25]
+    # one launch that repairs its output from its input cannot run in place, with either plan
+    one = tf.Plan(10, 4, 0, if_ft=1, if_err=1, own_scratch=False)
+    assert lib.tfft_exec_ws(one._h, x.data_ptr(), x.data_ptr(), None, 0) == -2

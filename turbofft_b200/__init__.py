@@ -44,13 +44,20 @@ def _lazy(x) -> bool:
 
 
 class Plan:
-    """One (logN, batch, dtype, FT mode) plan on one device."""
+    """One (logN, batch, dtype, FT mode) plan on one device.
+
+    Its intermediate buffer and its FT status belong to the plan, so its calls must not overlap: one
+    stream (or streams that wait for each other) and one host thread at a time.  fft() and ifft() have no
+    such limit: their plans bring a buffer per call."""
+
+    own_scratch = True  # False for the plans that fft() keeps: each call takes its buffer from torch's allocator
 
     def __init__(self, logN: int, batch: int, dtype: int = FLOAT2, if_ft: int = 0, if_err: int = 0,
                  thread_bs: int = 1, param_csv: Optional[str] = None, device: int = 0,
-                 single_pass: Optional[int] = None):
+                 single_pass: Optional[int] = None, own_scratch: bool = True):
         """single_pass = g asks for the one-kernel cluster plan with 2^g CTAs per cluster (-1 = the
-        size's default); None lets tfft_plan_create choose (built-in tables)."""
+        size's default); None lets tfft_plan_create choose (built-in tables).  own_scratch=False makes
+        a plan that holds no intermediate buffer (tfft_plan_create_ws)."""
         self._h = C.c_void_p()
         self.logN, self.batch, self.dtype = int(logN), int(batch), int(dtype)
         self.if_ft, self.if_err, self.thread_bs, self.device = int(bool(if_ft or if_err)), int(if_err), int(thread_bs), int(device)
@@ -59,8 +66,10 @@ class Plan:
                                                     self.thread_bs, self.device)
             _lib.check(rc, f"tfft_plan_create_single_pass(logN={logN}, batch={batch}, dtype={dtype}, log_cluster={single_pass})")
             return
-        rc = lib().tfft_plan_create(C.byref(self._h), self.logN, self.batch, self.dtype, int(if_ft), int(if_err),
-                                    self.thread_bs, param_csv.encode() if param_csv else None, self.device)
+        self.own_scratch = bool(own_scratch)
+        create = lib().tfft_plan_create if own_scratch else lib().tfft_plan_create_ws
+        rc = create(C.byref(self._h), self.logN, self.batch, self.dtype, int(if_ft), int(if_err),
+                    self.thread_bs, param_csv.encode() if param_csv else None, self.device)
         _lib.check(rc, f"tfft_plan_create(logN={logN}, batch={batch}, dtype={dtype}, ft={if_ft}, err={if_err})")
 
     def fuse_launches(self, log_chunk_signals: int, lag: int = 1) -> None:
@@ -108,7 +117,14 @@ class Plan:
         elif not (out.is_cuda and out.is_contiguous() and out.dtype == x.dtype and out.numel() == x.numel()) or _lazy(out):
             raise ValueError("bad output tensor")
         stream = torch.cuda.current_stream(x.device).cuda_stream
-        self.exec_ptr(x.data_ptr(), out.data_ptr(), stream)
+        if self.own_scratch:
+            self.exec_ptr(x.data_ptr(), out.data_ptr(), stream)
+        else:
+            # freed on return to the allocator, which gives it to later work of the same stream only
+            nbytes = lib().tfft_scratch_bytes(self._h)
+            ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device) if nbytes else None
+            _lib.check(lib().tfft_exec_ws(self._h, x.data_ptr(), out.data_ptr(), ws.data_ptr() if nbytes else None, stream),
+                       "tfft_exec_ws", self._h)
         return out
 
     def exec_host(self, x, out=None):
@@ -206,7 +222,8 @@ def _load_binding():
     _torch()  # the module's libtorch symbols
     from . import _torch_binding
 
-    entry = [C.cast(f, C.c_void_p).value for f in (lib().tfft_exec, lib().tfft_ft_status, lib().tfft_plan_info, lib().tfft_plan_shape)]
+    entry = [C.cast(getattr(lib(), "tfft_" + f), C.c_void_p).value
+             for f in ("exec", "ft_status", "plan_info", "plan_shape", "exec_ws", "scratch_bytes")]
     _torch_binding.bind(*entry, _plan_cache)
     _binding = _torch_binding
     return _binding
@@ -239,7 +256,7 @@ def _fft_strided(x, dim: int, norm, inverse: bool):
         _lib.check(lib().tfft_plan_create_strided(C.byref(plan._h), logn, inner, outer, plan.dtype, plan.device),
                    f"tfft_plan_create_strided(logN={logn}, inner={inner}, outer={outer})")
         plan.set_direction(inverse, float(n) ** expo)
-        _plan_cache[key] = plan
+        plan = _plan_cache.setdefault(key, plan)  # another thread may have made it meanwhile
     y = torch.empty_like(x)
     plan.exec_ptr(x.data_ptr(), y.data_ptr(), torch.cuda.current_stream(x.device).cuda_stream)
     return y
@@ -253,7 +270,7 @@ def fft(x, ft: bool = False, err: bool = False, thread_bs: int = 1, out=None, no
     the reference's --if_ft / --if_err.  norm follows torch.fft ("backward", "ortho", "forward");
     inverse=True is what ifft() calls.  dim other than the last axis runs the strided-batch plan
     (no copy, no transpose; lengths with a compiled strided-line kernel, FT off).  Plans are
-    cached per (device, shape, mode).
+    cached per (device, shape, mode); calls on different streams and from different threads may overlap.
     """
     expo = _NORM_FWD.get(norm)
     if expo is not None:
@@ -280,9 +297,9 @@ def fft(x, ft: bool = False, err: bool = False, thread_bs: int = 1, out=None, no
     key = (x.device.index, logn, batch, _dtype_code(x.dtype), bool(ft), bool(err), thread_bs, bool(inverse), expo)
     plan = _plan_cache.get(key)
     if plan is None:
-        plan = Plan(logn, batch, _dtype_code(x.dtype), int(ft or err), int(err), thread_bs, device=x.device.index)
+        plan = Plan(logn, batch, _dtype_code(x.dtype), int(ft or err), int(err), thread_bs, device=x.device.index, own_scratch=False)
         plan.set_direction(inverse, float(n) ** expo)
-        _plan_cache[key] = plan
+        plan = _plan_cache.setdefault(key, plan)
     y = plan(x.reshape(batch, n), out=None if out is None else out.reshape(batch, n))
     return y.reshape(x.shape)
 

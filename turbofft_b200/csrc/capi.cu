@@ -139,6 +139,7 @@ struct tfft_plan_s {
     int* pair_status = nullptr;
     long long pair_chunks = 0;
     int pair_log_chunk = 0, pair_lag = 1, pair_ring_chunks = 4, pair_grid = 0;
+    bool own_scratch = true;           // false: tfft_plan_create_ws, every exec brings its scratch
     void* scratch = nullptr;
     void* scratch2 = nullptr;          // 3-launch plans that correct: the middle launch writes here, so that
                                        // its own input survives for the recompute of a located tile
@@ -484,7 +485,7 @@ int launch_pair(tfft_plan p, const void* in, void* out, cudaStream_t st) {
 }
 
 template <typename T>
-int launch_all(tfft_plan p, const void* in, void* out, cudaStream_t st, void* scratch) {
+int launch_all(tfft_plan p, const void* in, void* out, cudaStream_t st, void* scratch, void* scratch2) {
     typedef typename Cplx<T>::type C;
     if (p->ck) return launch_cluster<T>(p, in, out, st);
     if (p->pk) return launch_pair<T>(p, in, out, st);
@@ -498,9 +499,9 @@ int launch_all(tfft_plan p, const void* in, void* out, cudaStream_t st, void* sc
         // launch scratch -> out.  A correcting plan recomputes a located tile from the launch's
         // input, so no launch may overwrite what it reads: its middle launch goes scratch ->
         // scratch2 (the reference alternates two buffers for every launch, main.cu:11-12).
-        const bool pingpong = p->scratch2 != nullptr;
-        a.in = (const C*)(i == 0 ? in : (i == 2 && pingpong ? p->scratch2 : scratch));
-        a.out = (C*)(i == p->n_launch - 1 ? out : (i == 1 && pingpong ? p->scratch2 : scratch));
+        const bool pingpong = scratch2 != nullptr;
+        a.in = (const C*)(i == 0 ? in : (i == 2 && pingpong ? scratch2 : scratch));
+        a.out = (C*)(i == p->n_launch - 1 ? out : (i == 1 && pingpong ? scratch2 : scratch));
         a.tw_st = (const C*)d.tw_st;
         a.tw_lo = (const C*)d.tw_lo;
         a.tw_hi = (const C*)d.tw_hi;
@@ -540,12 +541,13 @@ int launch_all(tfft_plan p, const void* in, void* out, cudaStream_t st, void* sc
     return TFFT_OK;
 }
 
-}  // namespace
+size_t batch_bytes(tfft_plan p) { return ((size_t)p->batch << p->logn) * p->esize(); }
 
-extern "C" {
+// three launches that repair by recomputing keep what the middle one reads (launch_all)
+bool needs_second_scratch(tfft_plan p) { return p->n_launch == 3 && p->if_err; }
 
-int tfft_plan_create(tfft_plan* plan, int logN, long long batch, int dtype, int if_ft, int if_err, int thread_bs,
-                     const char* param_csv, int device) {
+int create_plan(tfft_plan* plan, int logN, long long batch, int dtype, int if_ft, int if_err, int thread_bs,
+                const char* param_csv, int device, bool own_scratch) {
     if (!plan) return TFFT_ERR_BAD_ARG;
     *plan = nullptr;
     if (logN < 1 || logN > 30 || batch < 1 || (dtype != TFFT_FLOAT2 && dtype != TFFT_DOUBLE2) || thread_bs < 0 ||
@@ -590,6 +592,7 @@ int tfft_plan_create(tfft_plan* plan, int logN, long long batch, int dtype, int 
     p->inj_enable = p->if_err;
     p->thread_bs = thread_bs;
     p->device = device;
+    p->own_scratch = own_scratch;
     p->n_launch = row.launches;
     snprintf(p->nvtx_name, sizeof(p->nvtx_name), "tfft_exec logN=%d batch=%lld %s ft=%d", logN, batch,
              dtype == TFFT_FLOAT2 ? "c64" : "c128", p->if_ft + p->if_err);
@@ -667,11 +670,11 @@ int tfft_plan_create(tfft_plan* plan, int logN, long long batch, int dtype, int 
         const bool ok = dtype == TFFT_FLOAT2 ? build_tables<float>(p) : build_tables<double>(p);
         if (!ok) status = p->last_cuda_error ? TFFT_ERR_CUDA : TFFT_ERR_ALLOC;
     }
-    if (status == TFFT_OK && p->n_launch > 1) {
-        p->scratch = dev_alloc(p, ((size_t)batch << logN) * p->esize());
+    if (status == TFFT_OK && own_scratch && p->n_launch > 1) {
+        p->scratch = dev_alloc(p, batch_bytes(p));
         if (!p->scratch) status = TFFT_ERR_ALLOC;
-        if (status == TFFT_OK && p->n_launch == 3 && p->if_err) {
-            p->scratch2 = dev_alloc(p, ((size_t)batch << logN) * p->esize());
+        if (status == TFFT_OK && needs_second_scratch(p)) {
+            p->scratch2 = dev_alloc(p, batch_bytes(p));
             if (!p->scratch2) status = TFFT_ERR_ALLOC;
         }
     }
@@ -704,6 +707,23 @@ int tfft_plan_create(tfft_plan* plan, int logN, long long batch, int dtype, int 
     }
     *plan = p;
     return TFFT_OK;
+}
+
+// the located tile of a 1-launch plan is recomputed from the input
+bool needs_input_kept(tfft_plan p) { return p->n_launch == 1 && p->if_err && !(p->csum && csum_ok(p->L[0].k)); }
+
+}  // namespace
+
+extern "C" {
+
+int tfft_plan_create(tfft_plan* plan, int logN, long long batch, int dtype, int if_ft, int if_err, int thread_bs,
+                     const char* param_csv, int device) {
+    return create_plan(plan, logN, batch, dtype, if_ft, if_err, thread_bs, param_csv, device, true);
+}
+
+int tfft_plan_create_ws(tfft_plan* plan, int logN, long long batch, int dtype, int if_ft, int if_err, int thread_bs,
+                        const char* param_csv, int device) {
+    return create_plan(plan, logN, batch, dtype, if_ft, if_err, thread_bs, param_csv, device, false);
 }
 
 int tfft_plan_create_single_pass(tfft_plan* plan, int logN, long long batch, int dtype, int log_cluster, int thread_bs,
@@ -832,7 +852,7 @@ int tfft_plan_device_status(tfft_plan p, int* status) {
 int tfft_plan_fuse_launches(tfft_plan p, int log_chunk_signals, int lag) {
     if (!p || log_chunk_signals < 0 || log_chunk_signals > 20 || lag < 0 || lag > 2) return TFFT_ERR_BAD_ARG;
     if (p->pk) return TFFT_OK;
-    if (p->n_launch != 2 || p->if_ft || p->strided || p->ck) return TFFT_ERR_UNSUPPORTED;
+    if (p->n_launch != 2 || p->if_ft || p->strided || p->ck || !p->own_scratch) return TFFT_ERR_UNSUPPORTED;
     const LaunchDesc& a = p->L[0];
     const LaunchDesc& b = p->L[1];
     const PairKernel* pk = find_pair_kernel(p->dtype, a.logm, a.loge, a.logc, b.logm, b.loge, b.logc);
@@ -879,31 +899,37 @@ int tfft_plan_fuse_launches(tfft_plan p, int log_chunk_signals, int lag) {
 
 int tfft_plan_cluster_size(tfft_plan p) { return p ? (p->ck ? (1 << p->ck->logg) : 0) : TFFT_ERR_BAD_ARG; }
 
+static int run_plan(tfft_plan p, const void* in, void* out, void* scratch, void* scratch2, cudaStream_t st) {
+    NvtxRange range(p->nvtx_name);
+    return p->dtype == TFFT_FLOAT2 ? launch_all<float>(p, in, out, st, scratch, scratch2) : launch_all<double>(p, in, out, st, scratch, scratch2);
+}
+
 int tfft_exec(tfft_plan p, const void* in, void* out, void* stream) {
     if (!p || !in || !out) return TFFT_ERR_BAD_ARG;
-    if (in == out && p->n_launch == 1 && p->if_err && !(p->csum && csum_ok(p->L[0].k))) return TFFT_ERR_UNSUPPORTED;
+    if (in == out && needs_input_kept(p)) return TFFT_ERR_UNSUPPORTED;
+    if (!p->own_scratch && tfft_scratch_bytes(p)) return TFFT_ERR_UNSUPPORTED;
     DeviceGuard guard(p->device);
     if (!guard.ok) return TFFT_ERR_CUDA;
     cudaStream_t st = (cudaStream_t)stream;
     p->last_stream = st;
-    NvtxRange range(p->nvtx_name);
-    return p->dtype == TFFT_FLOAT2 ? launch_all<float>(p, in, out, st, p->scratch) : launch_all<double>(p, in, out, st, p->scratch);
+    return run_plan(p, in, out, p->scratch, p->scratch2, st);
 }
 
 size_t tfft_scratch_bytes(tfft_plan p) {
     if (!p || p->n_launch < 2 || p->ck || p->pk) return 0;  // single-pass and fused plans carry what they need
-    return ((size_t)p->batch << p->logn) * p->esize();
+    return batch_bytes(p) << (!p->own_scratch && needs_second_scratch(p) ? 1 : 0);
 }
 
 int tfft_exec_ws(tfft_plan p, const void* in, void* out, void* workspace, void* stream) {
     if (!p || !in || !out) return TFFT_ERR_BAD_ARG;
-    if (p->if_ft || p->pk) return TFFT_ERR_UNSUPPORTED;  // FT status buffers / the fused kernel's ring and counters belong to the plan: one exec at a time
+    // FT status buffers / the fused kernel's ring and counters belong to the plan: one exec at a time
+    if ((p->if_ft && p->own_scratch) || p->pk) return TFFT_ERR_UNSUPPORTED;
     if (tfft_scratch_bytes(p) && !workspace) return TFFT_ERR_BAD_ARG;
+    if (in == out && needs_input_kept(p)) return TFFT_ERR_UNSUPPORTED;
     DeviceGuard guard(p->device);
     if (!guard.ok) return TFFT_ERR_CUDA;
-    cudaStream_t st = (cudaStream_t)stream;
-    NvtxRange range(p->nvtx_name);
-    return p->dtype == TFFT_FLOAT2 ? launch_all<float>(p, in, out, st, workspace) : launch_all<double>(p, in, out, st, workspace);
+    void* second = needs_second_scratch(p) ? (char*)workspace + batch_bytes(p) : nullptr;
+    return run_plan(p, in, out, workspace, second, (cudaStream_t)stream);
 }
 
 // Pipelined form of tfft_exec_host for plans without FT whose batch spans several chunks:
@@ -1032,6 +1058,7 @@ static int exec_host_plain(tfft_plan p, const void* in_host, void* out_host, voi
 
 int tfft_exec_host(tfft_plan p, const void* in_host, void* out_host, void* stream) {
     if (!p || !in_host || !out_host) return TFFT_ERR_BAD_ARG;
+    if (!p->own_scratch) return TFFT_ERR_UNSUPPORTED;
     NvtxRange range("tfft_exec_host");
     DeviceGuard guard(p->device);
     if (!guard.ok) return TFFT_ERR_CUDA;
@@ -1042,6 +1069,7 @@ int tfft_exec_host(tfft_plan p, const void* in_host, void* out_host, void* strea
 
 int tfft_exec_host_async(tfft_plan p, const void* in_host, void* out_host, void* stream) {
     if (!p || !in_host || !out_host) return TFFT_ERR_BAD_ARG;
+    if (!p->own_scratch) return TFFT_ERR_UNSUPPORTED;
     NvtxRange range("tfft_exec_host_async");
     DeviceGuard guard(p->device);
     if (!guard.ok) return TFFT_ERR_CUDA;

@@ -4,14 +4,16 @@
 // A 16 x 1024-point transform keeps the GPU busy for 2.5 us; the interpreted form of this path
 // (attribute reads, a key tuple, reshape, ctypes argument conversion) kept the caller busy for 15.
 // Here a call reads the tensor's fields through ATen, looks the plan up in the SAME dictionary the
-// Python side keeps, allocates the output and calls tfft_exec.  Whatever is not an ordinary call --
+// Python side keeps, allocates the output and calls tfft_exec (Plan.__call__) or tfft_exec_ws (fft, ifft).  Whatever is not an ordinary call --
 // a plan that does not exist yet, a tensor that is not on a GPU, not contiguous, lazily conjugated, of
 // another type or length -- returns None, and the Python code does what it always did, errors included.
-// The module links nothing of the library: it is handed the address of the tfft_exec that _lib.py loaded.
+// The module links nothing of the library: it is handed the addresses of the entries that _lib.py loaded.
 #include <Python.h>
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -21,11 +23,15 @@
 namespace {
 
 typedef int (*ExecFn)(void*, const void*, void*, void*);
+typedef int (*ExecWsFn)(void*, const void*, void*, void*, void*);
+typedef size_t (*ScratchFn)(void*);
 typedef int (*StatusFn)(void*, int*, int*, int, int*, int, int*);
 typedef int (*InfoFn)(void*, int*);
 typedef int (*ShapeFn)(void*, int*, long long*, int*, int*);
 
 ExecFn g_exec = nullptr;
+ExecWsFn g_exec_ws = nullptr;
+ScratchFn g_scratch_bytes = nullptr;
 StatusFn g_status = nullptr;
 InfoFn g_info = nullptr;
 ShapeFn g_shape = nullptr;
@@ -59,7 +65,10 @@ void* plan_handle(PyObject* plan) {
 
 // Allocates the output (unless the caller brought one) and runs the plan on the current stream of the
 // tensor's device.  None when the library reports an error: the Python path repeats the call and raises.
-PyObject* execute(void* plan, const at::Tensor& x, PyObject* out_obj) {
+// shared: a plan of the cache, which callers on several streams and threads run at the same time; the intermediate
+// buffer is this call's own, from the caching allocator.  It goes back when the launches are queued and can then only
+// be given to later work of the same stream (and, inside a capture, of the same graph).
+PyObject* execute(void* plan, bool shared, const at::Tensor& x, PyObject* out_obj) {
     at::Tensor y;
     if (out_obj == Py_None) y = at::detail::empty_cuda(x.sizes(), x.scalar_type(), x.device(), c10::nullopt);
     else y = THPVariable_Unpack(out_obj);
@@ -67,8 +76,13 @@ PyObject* execute(void* plan, const at::Tensor& x, PyObject* out_obj) {
     int rc;
     const void* in = x.const_data_ptr();
     void* out = y.mutable_data_ptr();
+    at::DataPtr ws;
+    if (const size_t bytes = shared ? g_scratch_bytes(plan) : 0) {
+        c10::cuda::CUDAGuard guard(x.device());
+        ws = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
+    }
     Py_BEGIN_ALLOW_THREADS
-    rc = g_exec(plan, in, out, stream);
+    rc = shared ? g_exec_ws(plan, in, out, ws.get(), stream) : g_exec(plan, in, out, stream);
     Py_END_ALLOW_THREADS
     if (rc != 0) Py_RETURN_NONE;
     if (out_obj != Py_None) {
@@ -153,7 +167,7 @@ PyObject* fast_fft(PyObject*, PyObject* const* a, Py_ssize_t n) {
         void* h = plan_handle(plan);
         PyObject* r = nullptr;
         if (h) {
-            r = execute(h, x, a[4]);
+            r = execute(h, true, x, a[4]);
         } else {
             Py_INCREF(Py_None);
             r = Py_None;
@@ -181,7 +195,7 @@ PyObject* fast_exec(PyObject*, PyObject* const* a, Py_ssize_t n) {
             const at::Tensor& y = THPVariable_Unpack(a[2]);
             if (!y.is_cuda() || !y.is_contiguous() || y.scalar_type() != x.scalar_type() || y.numel() != x.numel()) Py_RETURN_NONE;
         }
-        return execute(h, x, a[2]);
+        return execute(h, false, x, a[2]);
     } catch (const std::exception& e) {
         PyErr_SetString(PyExc_RuntimeError, e.what());
         return nullptr;
@@ -213,24 +227,26 @@ PyObject* ft_status(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return PyLong_FromLong(rc);
 }
 
-// bind(addresses of tfft_exec, tfft_ft_status, tfft_plan_info and tfft_plan_shape, plan dictionary)
+// bind(addresses of tfft_exec, _ft_status, _plan_info, _plan_shape, _exec_ws and _scratch_bytes, plan dictionary)
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (n != 5 || !PyDict_Check(a[4])) {
-        PyErr_SetString(PyExc_TypeError, "bind(exec, ft_status, plan_info, plan_shape, dict)");
+    if (n != 7 || !PyDict_Check(a[6])) {
+        PyErr_SetString(PyExc_TypeError, "bind(exec, ft_status, plan_info, plan_shape, exec_ws, scratch_bytes, dict)");
         return nullptr;
     }
-    void* p[4];
-    for (int i = 0; i < 4; ++i) {
+    void* p[6];
+    for (int i = 0; i < 6; ++i) {
         p[i] = PyLong_AsVoidPtr(a[i]);
         if (!p[i] && PyErr_Occurred()) return nullptr;
     }
-    Py_INCREF(a[4]);
+    Py_INCREF(a[6]);
     Py_XDECREF(g_plans);
-    g_plans = a[4];
+    g_plans = a[6];
     g_exec = (ExecFn)p[0];
     g_status = (StatusFn)p[1];
     g_info = (InfoFn)p[2];
     g_shape = (ShapeFn)p[3];
+    g_exec_ws = (ExecWsFn)p[4];
+    g_scratch_bytes = (ScratchFn)p[5];
     Py_RETURN_NONE;
 }
 
