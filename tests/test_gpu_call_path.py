@@ -145,3 +145,36 @@ def test_plans_without_scratch_refuse_what_needs_it(torch_cuda):
     # one launch that repairs its output from its input cannot run in place, with either plan
     one = tf.Plan(10, 4, 0, if_ft=1, if_err=1, own_scratch=False)
     assert lib.tfft_exec_ws(one._h, x.data_ptr(), x.data_ptr(), None, 0) == -2
+
+
+@pytest.mark.parametrize("logn", [10, 18])
+def test_no_memory_is_reported_as_torch_reports_it(torch_cuda, logn):
+    """Programs catch torch.OutOfMemoryError to try a smaller batch; a call that ends so keeps no hold of its plan."""
+    import sys
+
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    x = torch.zeros((1 << 23) >> logn, 1 << logn, dtype=torch.complex64, device="cuda")  # 64 MiB
+    plan = tf.Plan(logn, x.shape[0], 0)
+    tf.fft(x), plan(x)
+    cached = next(p for k, p in tf._plan_cache.items() if k[:4] == (0, logn, x.shape[0], 0))
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    refs = sys.getrefcount(cached), sys.getrefcount(plan)
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (8 << 20)) / total)
+    held = []
+    try:
+        with pytest.raises(torch.OutOfMemoryError):  # what the allocator still has free in its segments
+            while True:
+                held.append(torch.empty(8 << 20, dtype=torch.uint8, device="cuda"))
+        for call in (lambda: tf.fft(x), lambda: plan(x)):
+            for _ in range(3):
+                with pytest.raises(torch.OutOfMemoryError):
+                    call()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+        del held
+    assert (sys.getrefcount(cached), sys.getrefcount(plan)) == refs
+    assert _same(torch, tf.fft(x), plan(x))
