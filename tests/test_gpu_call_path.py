@@ -178,3 +178,19 @@ def test_no_memory_is_reported_as_torch_reports_it(torch_cuda, logn):
         del held
     assert (sys.getrefcount(cached), sys.getrefcount(plan)) == refs
     assert _same(torch, tf.fft(x), plan(x))
+
+
+def test_whole_numbers_beyond_a_machine_word(torch_cuda):
+    """An axis is taken modulo the rank, a launch number modulo 2^32, whatever their size."""
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    x = torch.from_numpy(orc.make_input(16, 256, np.complex64, seed=4)).cuda()
+    for _ in range(2):
+        for dim in (-1, 0):
+            y = tf.fft(x, dim=dim)
+            assert all(_same(torch, tf.fft(x, dim=dim + k), y) for k in (1 << 40, 1 << 70, -(1 << 70)))
+    plan = tf.Plan(8, 16, 0, if_ft=1)
+    plan(x)
+    assert plan.ft_status(1 << 70) == plan.ft_status(0) == plan.ft_status()
+    assert plan.ft_status((1 << 70) - 1) == plan.ft_status(-1)

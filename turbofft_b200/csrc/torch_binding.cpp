@@ -131,7 +131,9 @@ PyObject* fast_fft(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor& x = THPVariable_Unpack(a[0]);
     const int code = type_code(x);
     const int64_t rank = x.dim();
-    int64_t dim = PyLong_AsLong(a[7]);
+    int overflow = 0;  // the Python path takes an axis of any size modulo the rank
+    int64_t dim = PyLong_AsLongLongAndOverflow(a[7], &overflow);
+    if (overflow) Py_RETURN_NONE;
     if (dim < 0) dim += rank;
     if (code < 0 || !x.is_cuda() || dim < 0 || dim >= rank || x.numel() == 0 || !x.is_contiguous()) Py_RETURN_NONE;
     const int64_t len = x.size(dim);
@@ -200,7 +202,7 @@ PyObject* ft_status(PyObject*, PyObject* const* a, Py_ssize_t n) {
         return nullptr;
     }
     void* h = plan_handle(a[0]);
-    const int launch = (int)PyLong_AsLong(a[1]);
+    const int launch = (int)PyLong_AsUnsignedLongLongMask(a[1]);  // as ctypes passes a C int
     int info[19] = {0}, nd = 0, nc = 0, nb = 0, rc = h ? g_info(h, info) : -1;
     if (rc == 0) {
         const int last = launch < 0 ? info[0] - 1 : launch;
