@@ -1,0 +1,46 @@
+"""tfft_ft_status against what may lie between the exec and the read: replayed graphs, totals over several execs, other
+plans and threads that wait, buffers that the call did not ask for."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from oracle import fft_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan(tf, logn=12, batch=64, tbs=4, err=1):
+    plan = tf.Plan(logn, batch, 0, if_ft=1, if_err=err, thread_bs=tbs)
+    plan.set_ft_params(1e5, 1000.0, 1e-3)
+    return plan
+
+
+def _input(torch, logn=12, batch=64):
+    return torch.from_numpy(orc.make_input(batch, 1 << logn, np.complex64, seed=logn + batch)).cuda()
+
+
+def _captured(torch, plan, x, inject):
+    plan.set_injection(inject)
+    y = torch.empty_like(x)
+    plan(x, y)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan(x, y)
+    torch.cuda.synchronize()
+    return graph
+
+
+def test_status_is_read_behind_replays_on_the_default_stream(torch_cuda):
+    """An exec captured on one stream and replayed on the default one, where it waits behind other work when the status is
+    asked for."""
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    plan, x = _plan(tf), _input(torch)
+    faulty, clean = _captured(torch, plan, x, True), _captured(torch, plan, x, False)
+    blocks = plan.info()[0]["grid"]
+    for graph, counts in ((faulty, (blocks, blocks)), (clean, (0, 0))) * 3:
+        torch.cuda._sleep(20_000_000)  # ten milliseconds on the default stream
+        graph.replay()
+        assert plan.ft_status()[:2] == counts

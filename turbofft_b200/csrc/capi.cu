@@ -1186,7 +1186,9 @@ int tfft_ft_status(tfft_plan p, int* n_detected, int* n_corrected, int launch, i
     if (!guard.ok) return TFFT_ERR_CUDA;
     if (launch < 0) launch = p->n_launch - 1;
     if (launch >= p->n_launch) return TFFT_ERR_BAD_ARG;
-    // One copy and one wait: the per-block results say which blocks detected and which tiles were repaired, so an
+    // The copy is on the default stream: a captured exec that was replayed there is not on last_stream, and a plain copy
+    // has always been behind it.  When the exec ran there too, its wait is the only one.
+    // The per-block results say which blocks detected and which tiles were repaired, so an
     // exec neither clears nor counts anything.  (Counters cleared by a memset before every exec, a wait and a copy
     // each for counters and blocks: 286 us for exec + status of 2^12 x 2^14 complex64 became 245 us.)
     const size_t blocks = ft_blocks(p), bytes = blocks * sizeof(int);
@@ -1199,8 +1201,9 @@ int tfft_ft_status(tfft_plan p, int* n_detected, int* n_corrected, int launch, i
         pageable.resize(blocks);
         host = pageable.data();
     }
-    if (!cuda_ok(p, cudaMemcpyAsync(host, p->ft_located, bytes, cudaMemcpyDeviceToHost, p->last_stream)) ||
-        !cuda_ok(p, cudaStreamSynchronize(p->last_stream)))
+    if (p->last_stream && !cuda_ok(p, cudaStreamSynchronize(p->last_stream))) return TFFT_ERR_CUDA;
+    if (!cuda_ok(p, cudaMemcpyAsync(host, p->ft_located, bytes, cudaMemcpyDeviceToHost, nullptr)) ||
+        !cuda_ok(p, cudaStreamSynchronize(nullptr)))
         return TFFT_ERR_CUDA;
     long long detected = 0, repaired = 0;
     if (p->ft_accumulate) {
