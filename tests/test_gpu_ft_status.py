@@ -44,3 +44,25 @@ def test_status_is_read_behind_replays_on_the_default_stream(torch_cuda):
         torch.cuda._sleep(20_000_000)  # ten milliseconds on the default stream
         graph.replay()
         assert plan.ft_status()[:2] == counts
+
+
+@pytest.mark.parametrize("logn,batch", [(12, 64), (18, 8)])
+def test_totals_over_replays_of_an_exec_captured_before(torch_cuda, logn, batch):
+    """set_ft_accumulate after the capture: the replays add up, and again from zero after each read."""
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    plan, x = _plan(tf, logn, batch), _input(torch, logn, batch)
+    graph = _captured(torch, plan, x, True)
+    graph.replay()
+    nd, nc = plan.ft_status()[:2]
+    assert nd == nc > 0
+    plan.set_ft_accumulate(True)
+    for n in (1, 3, 2):
+        for _ in range(n):
+            graph.replay()
+        assert plan.ft_status()[:2] == (n * nd, n * nc)
+    plan.set_ft_accumulate(False)
+    for _ in range(2):
+        graph.replay()
+    assert plan.ft_status()[:2] == (nd, nc)

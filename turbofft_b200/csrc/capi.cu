@@ -75,6 +75,11 @@ struct PipeSlots {
 };
 std::map<int, PipeSlots> g_pipe;
 
+// Counters of a plan and the word behind them, non-zero while ft_accumulate is set.  Blocks that detect something read it,
+// so that an exec captured before the switch counts when it is replayed after it, and the others spend no atomics: complex64
+// 2^1 x 2^26 with a fault in every block takes 1620 us when every exec counts.
+constexpr size_t kFtCounting = 6, kFtWords = 7;
+
 struct LaunchDesc {
     int role = 0, logm = 0, loge = 0, logc = 0;
     const KernelEntry* k = nullptr;
@@ -143,7 +148,7 @@ struct tfft_plan_s {
     void* scratch = nullptr;
     void* scratch2 = nullptr;          // 3-launch plans that correct: the middle launch writes here, so that
                                        // its own input survives for the recompute of a located tile
-    unsigned int* ft_count = nullptr;  // [3][2], counted only while ft_accumulate is set
+    unsigned int* ft_count = nullptr;  // [3][2], then the word that says whether execs count: kFtCounting
     int* ft_located = nullptr;         // the per-block results of all launches, one after the other
     unsigned long long* oob = nullptr;  // checked build: first out-of-range access of the last exec
     size_t owned_bytes = 0;
@@ -528,7 +533,8 @@ int launch_all(tfft_plan p, const void* in, void* out, cudaStream_t st, void* sc
         a.n_elems = p->batch << p->logn;
         a.oob = p->oob;
         a.ft_located = d.ft_located;
-        a.ft_count = p->ft_accumulate ? p->ft_count + 2 * i : nullptr;
+        a.ft_count = p->if_ft ? p->ft_count + 2 * i : nullptr;
+        a.ft_counting = p->if_ft ? p->ft_count + kFtCounting : nullptr;
         a.ft_diag = p->diag ? (T*)d.ft_diag : nullptr;
         void* args[] = {&a};
         const bool use_csum = ftmode == FT_CORRECT && p->csum && csum_ok(d.k);
@@ -685,11 +691,11 @@ int create_plan(tfft_plan* plan, int logN, long long batch, int dtype, int if_ft
     }
 #endif
     if (status == TFFT_OK && p->if_ft) {
-        p->ft_count = (unsigned int*)dev_alloc(p, 6 * sizeof(unsigned int));
+        p->ft_count = (unsigned int*)dev_alloc(p, kFtWords * sizeof(unsigned int));
         const size_t blocks = ft_blocks(p);
         p->ft_located = (int*)dev_alloc(p, blocks * sizeof(int));
         // tfft_ft_status before the first exec finds nothing detected
-        if (!p->ft_count || !p->ft_located || !cuda_ok(p, cudaMemset(p->ft_count, 0, 6 * sizeof(unsigned int))) ||
+        if (!p->ft_count || !p->ft_located || !cuda_ok(p, cudaMemset(p->ft_count, 0, kFtWords * sizeof(unsigned int))) ||
             !cuda_ok(p, cudaMemset(p->ft_located, 0xff, blocks * sizeof(int))))
             status = TFFT_ERR_ALLOC;
         size_t at = 0;
@@ -1231,10 +1237,14 @@ int tfft_ft_status(tfft_plan p, int* n_detected, int* n_corrected, int launch, i
 
 int tfft_set_ft_accumulate(tfft_plan p, int enable) {
     if (!p) return TFFT_ERR_BAD_ARG;
-    if (enable && !p->ft_accumulate && p->ft_count) {  // start the totals from zero
+    if ((enable != 0) != (p->ft_accumulate != 0) && p->ft_count) {
         DeviceGuard guard(p->device);
         if (!guard.ok) return TFFT_ERR_CUDA;
-        if (!cuda_ok(p, cudaStreamSynchronize(p->last_stream)) || !cuda_ok(p, cudaMemset(p->ft_count, 0, 6 * sizeof(unsigned int))))
+        // start the totals from zero; waited for, so that an exec on any stream finds them so
+        if (!cuda_ok(p, cudaStreamSynchronize(p->last_stream)) ||
+            !cuda_ok(p, cudaMemsetAsync(p->ft_count, 0, kFtCounting * sizeof(unsigned int), nullptr)) ||
+            !cuda_ok(p, cudaMemsetAsync(p->ft_count + kFtCounting, enable ? 1 : 0, sizeof(unsigned int), nullptr)) ||
+            !cuda_ok(p, cudaStreamSynchronize(nullptr)))
             return TFFT_ERR_CUDA;
     }
     p->ft_accumulate = enable ? 1 : 0;

@@ -101,7 +101,8 @@ struct KernelArgs {
     // intermediate is addressed, so that it lives in a ring of a few signals; 0 = whole buffer
     long long ring_clear;
     int* ft_located;          // per block: located tile iteration (1-based) or -1
-    unsigned int* ft_count;   // [0] blocks that detected, [1] tiles recomputed (null: the host counts from ft_located)
+    unsigned int* ft_count;   // [0] blocks that detected, [1] tiles recomputed; counted where *ft_counting is set
+    const unsigned int* ft_counting;
     T* ft_diag;               // per block: delta, S, delta_w (may be null)
 };
 
@@ -781,7 +782,7 @@ struct Fft {
                 if (fabs(delta) / (a.err_smoothing + fabs(mag)) > a.err_threshold) k = (int)round(fabs(dw) / fabs(delta));
                 s_k = k;
                 a.ft_located[blockIdx.x] = k;
-                if (k != -1 && a.ft_count) atomicAdd(a.ft_count, 1u);
+                if (k != -1 && *a.ft_counting) atomicAdd(a.ft_count, 1u);
                 if (a.ft_diag) {
                     a.ft_diag[3 * (long long)blockIdx.x + 0] = delta;
                     a.ft_diag[3 * (long long)blockIdx.x + 1] = mag;
@@ -796,7 +797,7 @@ struct Fft {
             if (k >= 1 && k <= done) {
                 A tin = acc_zero<A>(), tout = acc_zero<A>();
                 tile<false, false>(a, sm, blockIdx.x + (long long)(k - 1) * grid, false, f, tin, tout);
-                if (threadIdx.x == 0 && a.ft_count) atomicAdd(a.ft_count + 1, 1u);
+                if (threadIdx.x == 0 && *a.ft_counting) atomicAdd(a.ft_count + 1, 1u);
             }
         }
         if constexpr (FT == FT_CSUM) {
@@ -805,7 +806,7 @@ struct Fft {
             if (k >= 1 && k <= done) {
                 A tin = acc_zero<A>(), tout = acc_zero<A>();
                 tile<false, false, 2>(a, sm, blockIdx.x + (long long)(k - 1) * grid, false, f, tin, tout);
-                if (threadIdx.x == 0 && a.ft_count) atomicAdd(a.ft_count + 1, 1u);
+                if (threadIdx.x == 0 && *a.ft_counting) atomicAdd(a.ft_count + 1, 1u);
             }
         }
     }
