@@ -66,3 +66,33 @@ def test_totals_over_replays_of_an_exec_captured_before(torch_cuda, logn, batch)
     for _ in range(2):
         graph.replay()
     assert plan.ft_status()[:2] == (nd, nc)
+
+
+def test_a_status_read_that_waits_holds_up_no_other_plan(torch_cuda):
+    """One thread waits for a long queue on its stream; another plan's status is read meanwhile."""
+    import threading
+    import time
+
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    slow, quick, x = _plan(tf), _plan(tf), _input(torch)
+    busy, idle = torch.cuda.Stream(), torch.cuda.Stream()
+    blocks = quick.info()[0]["grid"]
+    for plan, stream in ((slow, busy), (quick, idle)):  # first reads, outside of what is timed
+        with torch.cuda.stream(stream):
+            plan(x)
+        plan.ft_status()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(1_500_000_000)  # most of a second
+        slow(x)
+    ended = []
+    waiter = threading.Thread(target=lambda: ended.append((slow.ft_status()[0], time.monotonic())))
+    waiter.start()
+    time.sleep(0.1)                       # the waiter is inside its call
+    with torch.cuda.stream(idle):
+        quick(x)
+    assert quick.ft_status()[0] == blocks
+    read = time.monotonic()
+    waiter.join()
+    assert ended[0][0] == blocks and read < ended[0][1] - 0.1

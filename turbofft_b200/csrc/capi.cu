@@ -149,6 +149,8 @@ struct tfft_plan_s {
     void* scratch2 = nullptr;          // 3-launch plans that correct: the middle launch writes here, so that
                                        // its own input survives for the recompute of a located tile
     unsigned int* ft_count = nullptr;  // [3][2], then the word that says whether execs count: kFtCounting
+    std::mutex status_mu;              // guards status_host: one status read of this plan at a time
+    int* status_host = nullptr;
     int* ft_located = nullptr;         // the per-block results of all launches, one after the other
     unsigned long long* oob = nullptr;  // checked build: first out-of-range access of the last exec
     size_t owned_bytes = 0;
@@ -389,11 +391,9 @@ void count_located(tfft_plan p, int i, const int* located, long long& detected, 
     }
 }
 
-// Pinned landing place of tfft_ft_status: a copy into pageable memory is staged by the driver and waits on its own.
-// One for all plans, made at the first call; longer results take the pageable route.
+// Up to this size tfft_ft_status lands in a pinned buffer of the plan, made at the first call: a copy into pageable
+// memory is staged by the driver and waits on its own.
 constexpr size_t kStatusBytes = 64u << 10;
-std::mutex g_status_mu;
-int* g_status_host = nullptr;
 
 // Launches one fft_kernel with the programmatic-dependent-launch attribute (fft_kernels.cuh,
 // wait_for_previous_launch): its blocks are placed while the launch before it drains, where the
@@ -1199,14 +1199,10 @@ int tfft_ft_status(tfft_plan p, int* n_detected, int* n_corrected, int launch, i
     // each for counters and blocks: 286 us for exec + status of 2^12 x 2^14 complex64 became 245 us.)
     const size_t blocks = ft_blocks(p), bytes = blocks * sizeof(int);
     std::vector<int> pageable;
-    std::unique_lock<std::mutex> lock(g_status_mu);
-    if (!g_status_host && !cuda_ok(p, cudaHostAlloc((void**)&g_status_host, kStatusBytes, cudaHostAllocPortable))) return TFFT_ERR_CUDA;
-    int* host = g_status_host;
-    if (bytes > kStatusBytes) {
-        lock.unlock();
-        pageable.resize(blocks);
-        host = pageable.data();
-    }
+    std::lock_guard<std::mutex> lock(p->status_mu);
+    if (bytes > kStatusBytes) pageable.resize(blocks);
+    else if (!p->status_host && !cuda_ok(p, cudaHostAlloc((void**)&p->status_host, bytes, cudaHostAllocPortable))) return TFFT_ERR_CUDA;
+    int* host = bytes > kStatusBytes ? pageable.data() : p->status_host;
     if (p->last_stream && !cuda_ok(p, cudaStreamSynchronize(p->last_stream))) return TFFT_ERR_CUDA;
     if (!cuda_ok(p, cudaMemcpyAsync(host, p->ft_located, bytes, cudaMemcpyDeviceToHost, nullptr)) ||
         !cuda_ok(p, cudaStreamSynchronize(nullptr)))
@@ -1309,6 +1305,7 @@ int tfft_plan_destroy(tfft_plan p) {
     if (p->chunk_plan) tfft_plan_destroy(p->chunk_plan);
     if (p->tail_plan) tfft_plan_destroy(p->tail_plan);
     for (void* q : p->allocs) cudaFree(q);
+    if (p->status_host) cudaFreeHost(p->status_host);
     delete p;
     return TFFT_OK;
 }
