@@ -96,3 +96,46 @@ def test_a_status_read_that_waits_holds_up_no_other_plan(torch_cuda):
     read = time.monotonic()
     waiter.join()
     assert ended[0][0] == blocks and read < ended[0][1] - 0.1
+
+
+@pytest.mark.parametrize("logn,batch,tbs,total", [(12, 64, 4, False), (12, 64, 4, True), (7, 1 << 18, 1, False), (7, 1 << 18, 1, True),
+                                                  (18, 40, 2, False), (18, 40, 2, True), (22, 3, 2, True)])
+def test_every_form_of_the_call_gives_the_same_answer(torch_cuda, logn, batch, tbs, total):
+    """Counts alone, counts with the blocks of one launch, a buffer that is too short, nothing at all; results on both
+    sides of the size that is read through pinned memory; totals are cleared by each read."""
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    plan, x = _plan(tf, logn, batch, tbs), _input(torch, logn, batch)
+    lib, info = tf.lib(), plan.info()
+    stream = torch.cuda.Stream()  # not ordered with the default stream by itself
+    stream.wait_stream(torch.cuda.current_stream())
+    plan.set_injection(True, launch=0)
+    plan.set_ft_accumulate(total)
+
+    def status(launch, cap, counts=True, blocks=True):
+        with torch.cuda.stream(stream):
+            for _ in range(2):
+                plan(x)
+        nd, nc, nb = C.c_int(-7), C.c_int(-7), C.c_int(-7)
+        loc = (C.c_int * max(cap, 1))(*[-7] * max(cap, 1))
+        rc = lib.tfft_ft_status(plan._h, C.byref(nd) if counts else None, C.byref(nc) if counts else None, launch,
+                                loc if cap else None, cap, C.byref(nb) if blocks else None)
+        assert rc == 0
+        return nd.value, nc.value, nb.value, list(loc)[:cap]
+
+    grids = [l["grid"] for l in info]
+    runs = 2 if total else 1
+    want = (runs * grids[0], runs * grids[0])
+    for launch in range(len(info)):
+        nd, nc, nb, loc = status(launch, grids[launch])
+        assert (nd, nc, nb) == (*want, grids[launch])
+        assert all((k != -1) == (launch == 0) for k in loc)
+        short = max(1, grids[launch] // 3)
+        assert status(launch, short)[3] == loc[:short]
+        assert status(launch, 0)[:3] == (*want, grids[launch])
+        assert status(launch, grids[launch], counts=False, blocks=False)[3] == loc
+    assert status(-1, 0, counts=False, blocks=False)[:3] == (-7, -7, -7)
+    plan.set_injection(False)
+    assert status(0, grids[0])[:2] == (0, 0)
+    assert lib.tfft_ft_status(plan._h, None, None, len(info), None, 0, None) == -1

@@ -1192,38 +1192,40 @@ int tfft_ft_status(tfft_plan p, int* n_detected, int* n_corrected, int launch, i
     if (!guard.ok) return TFFT_ERR_CUDA;
     if (launch < 0) launch = p->n_launch - 1;
     if (launch >= p->n_launch) return TFFT_ERR_BAD_ARG;
-    // The copy is on the default stream: a captured exec that was replayed there is not on last_stream, and a plain copy
+    // The copies are on the default stream: a captured exec that was replayed there is not on last_stream, and a plain copy
     // has always been behind it.  When the exec ran there too, its wait is the only one.
-    // The per-block results say which blocks detected and which tiles were repaired, so an
-    // exec neither clears nor counts anything.  (Counters cleared by a memset before every exec, a wait and a copy
+    // What is fetched is what is needed: the plan's counters while they add up, else the per-block results of all
+    // launches, which say which blocks detected and which tiles were repaired, so that an exec neither clears nor counts
+    // anything; of those, the blocks of one launch while the counters add up and the caller asks for them.
+    // (Counters cleared by a memset before every exec, a wait and a copy
     // each for counters and blocks: 286 us for exec + status of 2^12 x 2^14 complex64 became 245 us.)
-    const size_t blocks = ft_blocks(p), bytes = blocks * sizeof(int);
+    const bool totals = p->ft_accumulate != 0;
+    const size_t asked = located && cap > 0 ? (size_t)p->L[launch].grid : 0;
+    const size_t blocks = totals ? asked : ft_blocks(p);
+    const int* src = totals ? p->L[launch].ft_located : p->ft_located;
+    const size_t words = kFtCounting + blocks;
     std::vector<int> pageable;
     std::lock_guard<std::mutex> lock(p->status_mu);
-    if (bytes > kStatusBytes) pageable.resize(blocks);
-    else if (!p->status_host && !cuda_ok(p, cudaHostAlloc((void**)&p->status_host, bytes, cudaHostAllocPortable))) return TFFT_ERR_CUDA;
-    int* host = bytes > kStatusBytes ? pageable.data() : p->status_host;
+    if (words * sizeof(int) > kStatusBytes) pageable.resize(words);
+    else if (!p->status_host && !cuda_ok(p, cudaHostAlloc((void**)&p->status_host, kStatusBytes, cudaHostAllocPortable))) return TFFT_ERR_CUDA;
+    int* host = pageable.empty() ? p->status_host : pageable.data();
+    int* l = host + kFtCounting;
     if (p->last_stream && !cuda_ok(p, cudaStreamSynchronize(p->last_stream))) return TFFT_ERR_CUDA;
-    if (!cuda_ok(p, cudaMemcpyAsync(host, p->ft_located, bytes, cudaMemcpyDeviceToHost, nullptr)) ||
-        !cuda_ok(p, cudaStreamSynchronize(nullptr)))
+    if (blocks && !cuda_ok(p, cudaMemcpyAsync(l, src, blocks * sizeof(int), cudaMemcpyDeviceToHost, nullptr))) return TFFT_ERR_CUDA;
+    if (totals && (!cuda_ok(p, cudaMemcpyAsync(host, p->ft_count, kFtCounting * sizeof(int), cudaMemcpyDeviceToHost, nullptr)) ||
+                   !cuda_ok(p, cudaMemsetAsync(p->ft_count, 0, kFtCounting * sizeof(int), nullptr))))
         return TFFT_ERR_CUDA;
+    if (!cuda_ok(p, cudaStreamSynchronize(nullptr))) return TFFT_ERR_CUDA;  // the clear too: the next exec may be on any stream
     long long detected = 0, repaired = 0;
-    if (p->ft_accumulate) {
-        unsigned int cnt[6];
-        if (!cuda_ok(p, cudaMemcpy(cnt, p->ft_count, sizeof(cnt), cudaMemcpyDeviceToHost)) ||
-            !cuda_ok(p, cudaMemset(p->ft_count, 0, sizeof(cnt))))
-            return TFFT_ERR_CUDA;
-        for (int i = 0; i < p->n_launch; ++i) {
-            detected += cnt[2 * i];
-            repaired += cnt[2 * i + 1];
-        }
-    }
-    const int* l = host;
     for (int i = 0; i < p->n_launch; ++i) {
-        if (!p->ft_accumulate) count_located(p, i, l, detected, repaired);
-        if (i == launch && located && cap > 0)
-            memcpy(located, l, (size_t)(cap < (int)p->L[i].grid ? cap : (int)p->L[i].grid) * sizeof(int));
-        l += p->L[i].grid;
+        if (totals) {
+            detected += (unsigned)host[2 * i];
+            repaired += (unsigned)host[2 * i + 1];
+        } else {
+            count_located(p, i, l, detected, repaired);
+        }
+        if (i == launch && asked) memcpy(located, l, ((size_t)cap < asked ? (size_t)cap : asked) * sizeof(int));
+        if (!totals) l += p->L[i].grid;
     }
     if (n_detected) *n_detected = (int)detected;
     if (n_corrected) *n_corrected = (int)repaired;
