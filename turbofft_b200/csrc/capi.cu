@@ -338,6 +338,10 @@ bool build_cluster_tables(tfft_plan p) {
     return true;
 }
 
+// Table uploads (the last part of a copy from pageable memory) and clears may still be under way on the default stream when
+// their calls return; an exec on a stream that does not wait for that one has to find them done.
+bool setup_done(tfft_plan p) { return cuda_ok(p, cudaStreamSynchronize(nullptr)); }
+
 int ilog2_exact(long long x) {
     int l = 0;
     while ((1LL << l) < x) ++l;
@@ -706,6 +710,7 @@ int create_plan(tfft_plan* plan, int logN, long long batch, int dtype, int if_ft
             if (!p->L[i].ft_diag) status = TFFT_ERR_ALLOC;
         }
     }
+    if (status == TFFT_OK && !setup_done(p)) status = TFFT_ERR_CUDA;
     if (status != TFFT_OK) {
         for (void* q : p->allocs) cudaFree(q);
         delete p;
@@ -767,6 +772,7 @@ int tfft_plan_create_single_pass(tfft_plan* plan, int logN, long long batch, int
         p->cstatus = (int*)dev_alloc(p, sizeof(int));
         ok = p->cstatus && cuda_ok(p, cudaMemset(p->cstatus, 0, sizeof(int)));
     }
+    ok = ok && setup_done(p);
     if (!ok) {
         const int status = p->last_cuda_error ? TFFT_ERR_CUDA : TFFT_ERR_ALLOC;
         for (void* q : p->allocs) cudaFree(q);
@@ -835,6 +841,7 @@ int tfft_plan_create_strided(tfft_plan* plan, int logN, long long inner, long lo
         if (!p->oob || !cuda_ok(p, cudaMemset(p->oob, 0, sizeof(unsigned long long)))) status = TFFT_ERR_ALLOC;
     }
 #endif
+    if (status == TFFT_OK && !setup_done(p)) status = TFFT_ERR_CUDA;
     if (status != TFFT_OK) {
         for (void* q : p->allocs) cudaFree(q);
         delete p;
@@ -878,7 +885,7 @@ int tfft_plan_fuse_launches(tfft_plan p, int log_chunk_signals, int lag) {
     unsigned int* done = (unsigned int*)dev_alloc(p, (size_t)(2 * chunks + 2) * sizeof(unsigned int));
     int* status = (int*)dev_alloc(p, sizeof(int));
     if (!ring || !done || !status) return TFFT_ERR_ALLOC;  // the plan keeps what was allocated until it is destroyed
-    if (!cuda_ok(p, cudaMemset(status, 0, sizeof(int)))) return TFFT_ERR_CUDA;
+    if (!cuda_ok(p, cudaMemset(status, 0, sizeof(int))) || !setup_done(p)) return TFFT_ERR_CUDA;
     // the launches' whole-batch intermediate is not needed any more
     if (p->scratch) {
         for (size_t i = 0; i < p->allocs.size(); ++i)
@@ -1265,7 +1272,7 @@ int tfft_bounds_status(tfft_plan p, long long* bad_index, int* site) {
         if (idx & (1LL << 55)) idx |= ~((1LL << 56) - 1);  // sign of a negative index
         if (bad_index) *bad_index = idx;
         if (site) *site = (int)((w >> 56) & 0x7f);
-        if (!cuda_ok(p, cudaMemset(p->oob, 0, sizeof(w)))) return TFFT_ERR_CUDA;
+        if (!cuda_ok(p, cudaMemset(p->oob, 0, sizeof(w))) || !setup_done(p)) return TFFT_ERR_CUDA;
         return 1;
     }
     return TFFT_OK;
