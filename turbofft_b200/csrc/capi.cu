@@ -958,6 +958,7 @@ static int exec_host_pipelined(tfft_plan p, const void* in_host, void* out_host,
     // chunk plans are ordinary launch plans over whole signals: strided-batch, single-pass and fused plans
     // (and FT plans, whose status is per plan) take the unchunked path with their own kernels
     if (p->if_ft || p->strided || p->ck || p->pk || cb < 1 || p->batch < 3 * cb) return TFFT_ERR_UNSUPPORTED;
+    std::lock_guard<std::mutex> lock(g_stage_mu);  // the sub-plans too: two threads may bring the first calls of one plan
     if (!p->pipe_ready) {
         // every resource is created only if it is still missing, so a call that failed half way
         // can be repeated; the plan's destructor releases whatever exists
@@ -977,7 +978,6 @@ static int exec_host_pipelined(tfft_plan p, const void* in_host, void* out_host,
     }
     cb = p->chunk_batch;
     const size_t chunk_bytes = (size_t)cb * sig_bytes;
-    std::lock_guard<std::mutex> lock(g_stage_mu);
     PipeSlots& ps = g_pipe[p->device];
     if (!ps.ready) {
         for (int i = 0; i < 3; ++i) {
