@@ -136,7 +136,8 @@ int tfft_plan_create_ws(tfft_plan* plan, int logN, long long batch, int dtype, i
  * (initializeData.h:39, main.cu:72).  Plans without FT whose batch spans at least
  * three chunks (a sixteenth of the batch, 2 to 64 MiB of whole signals, or one signal of up to 512 MiB) are pipelined: chunks of whole signals are copied in,
  * transformed and copied out on three internal streams so both PCIe directions
- * overlap the kernels (use pinned host buffers).  Device staging buffers, the
+ * overlap the kernels (use pinned host buffers).  in_host and out_host may be the same, or overlap
+ * in part (then the batch travels in one piece).  Device staging buffers, the
  * three streams and their events are per device, grow-only, shared by all plans
  * and kept until the library is unloaded; calls are serialised. */
 int tfft_exec_host(tfft_plan plan, const void* in_host, void* out_host, void* stream);

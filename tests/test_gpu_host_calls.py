@@ -35,3 +35,27 @@ def test_first_calls_of_one_plan_from_several_threads(torch_cuda, logn, batch):
         [t.start() for t in threads]
         [t.join() for t in threads]
         assert all(_same(torch, g, w) for g, w in zip(got, want))
+
+
+@pytest.mark.parametrize("logn,batch", [(10, 1001), (16, 40)])
+@pytest.mark.parametrize("shift", [0, 1, -1, 5, -5])
+@pytest.mark.parametrize("asynchronous", [False, True])
+def test_buffers_that_share_memory(torch_cuda, logn, batch, shift, asynchronous):
+    """The input is read before the output lands on it, wherever the two lie in one array (shift in signals)."""
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    x = torch.from_numpy(orc.make_input(batch, 1 << logn, np.complex64, seed=logn))
+    plan = tf.Plan(logn, batch, 0)
+    want = plan(x.cuda()).cpu()
+    both = torch.zeros(batch + abs(shift), 1 << logn, dtype=x.dtype).pin_memory()
+    src = both[max(0, -shift):][:batch]
+    dst = both[max(0, shift):][:batch]
+    for _ in range(2):
+        src.copy_(x)
+        if asynchronous:
+            plan.exec_host_async(src, dst)
+            tf.host_sync()
+        else:
+            plan.exec_host(src, dst)
+        assert _same(torch, dst, want)

@@ -958,6 +958,9 @@ static int exec_host_pipelined(tfft_plan p, const void* in_host, void* out_host,
     // chunk plans are ordinary launch plans over whole signals: strided-batch, single-pass and fused plans
     // (and FT plans, whose status is per plan) take the unchunked path with their own kernels
     if (p->if_ft || p->strided || p->ck || p->pk || cb < 1 || p->batch < 3 * cb) return TFFT_ERR_UNSUPPORTED;
+    // buffers that overlap in part: a chunk's results would land on input that a later chunk has yet to read
+    const uintptr_t src0 = (uintptr_t)in_host, dst0 = (uintptr_t)out_host, span = (uintptr_t)p->batch * sig_bytes;
+    if (src0 != dst0 && src0 < dst0 + span && dst0 < src0 + span) return TFFT_ERR_UNSUPPORTED;
     std::lock_guard<std::mutex> lock(g_stage_mu);  // the sub-plans too: two threads may bring the first calls of one plan
     if (!p->pipe_ready) {
         // every resource is created only if it is still missing, so a call that failed half way
