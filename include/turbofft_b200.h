@@ -134,9 +134,10 @@ int tfft_plan_create_ws(tfft_plan* plan, int logN, long long batch, int dtype, i
  * tfft_exec and copies the result back, then synchronises.  Replaces the
  * cudaMemcpy pair around the launches in initializeData()/test_turbofft()
  * (initializeData.h:39, main.cu:72).  Plans without FT whose batch spans at least
- * three chunks (a sixteenth of the batch, 2 to 64 MiB of whole signals, or one signal of up to 512 MiB) are pipelined: chunks of whole signals are copied in,
+ * three chunks (page-locked buffers: a sixteenth of the batch, 2 to 64 MiB of whole signals; others 64 MiB; in either case
+ * at least one signal, of up to 512 MiB) are pipelined: chunks of whole signals are copied in,
  * transformed and copied out on three internal streams so both PCIe directions
- * overlap the kernels (use pinned host buffers).  in_host and out_host may be the same, or overlap
+ * overlap the kernels (use page-locked host buffers).  in_host and out_host may be the same, or overlap
  * in part (then the batch travels in one piece).  Device staging buffers, the
  * three streams and their events are per device, grow-only, shared by all plans
  * and kept until the library is unloaded; calls are serialised. */

@@ -59,3 +59,19 @@ def test_buffers_that_share_memory(torch_cuda, logn, batch, shift, asynchronous)
         else:
             plan.exec_host(src, dst)
         assert _same(torch, dst, want)
+
+
+@pytest.mark.parametrize("logn,batch", [(12, 1000), (12, 6500), (18, 100)])  # 31 and 203 MiB, 200 MiB of longer signals
+def test_page_locked_and_ordinary_buffers_alternate_on_one_plan(torch_cuda, logn, batch):
+    """They are cut differently (ordinary buffers not at all below three chunks of 64 MiB), each with plans of its own
+    that follow a change of direction."""
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    x = torch.from_numpy(orc.make_input(batch, 1 << logn, np.complex64, seed=logn))
+    locked, plan = x.pin_memory(), tf.Plan(logn, batch, 0)
+    for inverse in (False, True, False):
+        plan.set_direction(inverse, 0.5)
+        want = plan(x.cuda()).cpu()
+        for src, dst in ((x, torch.empty_like(x)), (locked, torch.empty_like(x).pin_memory()), (locked, torch.empty_like(x)), (x, None)):
+            assert _same(torch, plan.exec_host(src, dst), want)

@@ -56,10 +56,19 @@ std::map<int, StagePair> g_stage;
 // gain beyond, and six slots of that size are held) and at least 2 MiB (40 us of copying, which covers the dozen driver
 // calls that queue a chunk).  Bound: PCIe.  2^12 x 2^12 complex64 (128 MiB each way), which chunks of 64 MiB left
 // unpipelined: 4.84 -> 3.21 ms.
+// Buffers that are not page locked gain nothing from many chunks: their copies are staged by the driver inside the call, so
+// a copy out keeps the next copy in from being queued.  They take the largest chunk, with which a call of under three is
+// not cut at all: 2^12 x 2^9 (16 MiB each way) 1693 us in one piece, 2146 in eight; 2^12 x 2^12 18.2 ms against 19.2.
 constexpr size_t kPipeChunkMost = 64u << 20, kPipeChunkLeast = 2u << 20;
-size_t pipe_chunk_bytes(size_t call_bytes) {
-    const size_t want = call_bytes / 16;
+size_t pipe_chunk_bytes(size_t call_bytes, bool locked) {
+    const size_t want = locked ? call_bytes / 16 : kPipeChunkMost;
     return want < kPipeChunkLeast ? kPipeChunkLeast : (want > kPipeChunkMost ? kPipeChunkMost : want);
+}
+bool page_locked(const void* host) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, host) == cudaSuccess) return a.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return false;
 }
 struct PipeSlots {
     void* in[3] = {nullptr, nullptr, nullptr};
@@ -98,6 +107,14 @@ struct LaunchDesc {
     void* cks = nullptr;
     int* ft_located = nullptr;
     void* ft_diag = nullptr;
+};
+
+// Sub-plans of the pipelined host path: for one chunk and for the ragged last one
+struct ChunkPlans {
+    tfft_plan chunk = nullptr;
+    tfft_plan tail = nullptr;
+    long long batch = 0;  // signals per chunk
+    bool ready = false;
 };
 
 struct DeviceGuard {
@@ -169,12 +186,7 @@ struct tfft_plan_s {
     std::vector<void*> allocs;
     std::string param_csv;            // empty = built-in table
     char nvtx_name[64] = "tfft_exec";  // range name of this plan's execs
-    // host-buffer pipeline (tfft_exec_host): sub-plans for one chunk / the ragged last chunk,
-    // three internal streams and per-slot events
-    tfft_plan chunk_plan = nullptr;
-    tfft_plan tail_plan = nullptr;
-    long long chunk_batch = 0;
-    bool pipe_ready = false;  // the sub-plans of the pipelined host path exist
+    ChunkPlans pipe[2];  // host-buffer pipeline (tfft_exec_host): [0] buffers that are not page locked, [1] page-locked ones
     size_t esize() const { return dtype == TFFT_FLOAT2 ? sizeof(float2) : sizeof(double2); }
 };
 
@@ -952,7 +964,8 @@ int tfft_exec_ws(tfft_plan p, const void* in, void* out, void* workspace, void* 
 // not qualify (the caller then takes the plain path).
 static int exec_host_pipelined(tfft_plan p, const void* in_host, void* out_host, cudaStream_t user, bool sync) {
     const size_t sig_bytes = ((size_t)1 << p->logn) * p->esize();
-    long long cb = (long long)(pipe_chunk_bytes((size_t)p->batch * sig_bytes) / sig_bytes);
+    const bool locked = page_locked(in_host) && page_locked(out_host);
+    long long cb = (long long)(pipe_chunk_bytes((size_t)p->batch * sig_bytes, locked) / sig_bytes);
     // signals longer than a chunk travel one per chunk (up to 512 MiB each: six staging slots of that size)
     if (cb < 1 && sig_bytes <= ((size_t)512 << 20)) cb = 1;
     // chunk plans are ordinary launch plans over whole signals: strided-batch, single-pass and fused plans
@@ -962,24 +975,23 @@ static int exec_host_pipelined(tfft_plan p, const void* in_host, void* out_host,
     const uintptr_t src0 = (uintptr_t)in_host, dst0 = (uintptr_t)out_host, span = (uintptr_t)p->batch * sig_bytes;
     if (src0 != dst0 && src0 < dst0 + span && dst0 < src0 + span) return TFFT_ERR_UNSUPPORTED;
     std::lock_guard<std::mutex> lock(g_stage_mu);  // the sub-plans too: two threads may bring the first calls of one plan
-    if (!p->pipe_ready) {
+    ChunkPlans& cp = p->pipe[locked ? 1 : 0];
+    if (!cp.ready) {
         // every resource is created only if it is still missing, so a call that failed half way
         // can be repeated; the plan's destructor releases whatever exists
         const char* csv = p->param_csv.empty() ? nullptr : p->param_csv.c_str();
-        if (!p->chunk_plan) {
-            const int rc = tfft_plan_create(&p->chunk_plan, p->logn, cb, p->dtype, 0, 0, p->thread_bs, csv, p->device);
+        if (!cp.chunk) {
+            const int rc = tfft_plan_create(&cp.chunk, p->logn, cb, p->dtype, 0, 0, p->thread_bs, csv, p->device);
             if (rc != TFFT_OK) return rc;
-            p->chunk_batch = cb;
+            cp.batch = cb;
         }
-        if (p->batch % p->chunk_batch && !p->tail_plan) {
-            const int rc = tfft_plan_create(&p->tail_plan, p->logn, p->batch % p->chunk_batch, p->dtype, 0, 0,
-                                            p->thread_bs, csv, p->device);
+        if (p->batch % cp.batch && !cp.tail) {
+            const int rc = tfft_plan_create(&cp.tail, p->logn, p->batch % cp.batch, p->dtype, 0, 0, p->thread_bs, csv, p->device);
             if (rc != TFFT_OK) return rc;
         }
         tfft_set_direction(p, p->inverse, p->scale);  // hand the direction down to the sub-plans
-        p->pipe_ready = true;
+        cp.ready = true;
     }
-    cb = p->chunk_batch;
     const size_t chunk_bytes = (size_t)cb * sig_bytes;
     PipeSlots& ps = g_pipe[p->device];
     if (!ps.ready) {
@@ -1033,7 +1045,7 @@ static int exec_host_pipelined(tfft_plan p, const void* in_host, void* out_host,
         if (!cuda_ok(p, cudaMemcpyAsync(ps.in[slot], src, bytes, cudaMemcpyHostToDevice, s_in))) return TFFT_ERR_CUDA;
         if (!cuda_ok(p, cudaEventRecord(ps.ev_in[slot], s_in))) return TFFT_ERR_CUDA;
         if (!cuda_ok(p, cudaStreamWaitEvent(s_fft, ps.ev_in[slot], 0))) return TFFT_ERR_CUDA;
-        const int rc = tfft_exec(this_b == cb ? p->chunk_plan : p->tail_plan, ps.in[slot], ps.out[slot], s_fft);
+        const int rc = tfft_exec(this_b == cb ? cp.chunk : cp.tail, ps.in[slot], ps.out[slot], s_fft);
         if (rc != TFFT_OK) return rc;
         if (!cuda_ok(p, cudaEventRecord(ps.ev_fft[slot], s_fft))) return TFFT_ERR_CUDA;
         if (!cuda_ok(p, cudaStreamWaitEvent(s_out, ps.ev_fft[slot], 0))) return TFFT_ERR_CUDA;
@@ -1178,8 +1190,10 @@ int tfft_set_direction(tfft_plan p, int inverse, double scale) {
     if (!p || !(scale == scale)) return TFFT_ERR_BAD_ARG;
     p->inverse = inverse ? 1 : 0;
     p->scale = scale;
-    if (p->chunk_plan) tfft_set_direction(p->chunk_plan, inverse, scale);
-    if (p->tail_plan) tfft_set_direction(p->tail_plan, inverse, scale);
+    for (ChunkPlans& cp : p->pipe) {
+        if (cp.chunk) tfft_set_direction(cp.chunk, inverse, scale);
+        if (cp.tail) tfft_set_direction(cp.tail, inverse, scale);
+    }
     return TFFT_OK;
 }
 
@@ -1313,9 +1327,11 @@ int tfft_ft_diag(tfft_plan p, int launch, double* diag, int cap_blocks) {
 int tfft_plan_destroy(tfft_plan p) {
     if (!p) return TFFT_ERR_BAD_ARG;
     DeviceGuard guard(p->device);
-    if (p->pipe_ready) tfft_host_sync(p->device);  // chunks this plan queued with tfft_exec_host_async still use its sub-plans
-    if (p->chunk_plan) tfft_plan_destroy(p->chunk_plan);
-    if (p->tail_plan) tfft_plan_destroy(p->tail_plan);
+    if (p->pipe[0].ready || p->pipe[1].ready) tfft_host_sync(p->device);  // chunks this plan queued with tfft_exec_host_async still use its sub-plans
+    for (ChunkPlans& cp : p->pipe) {
+        if (cp.chunk) tfft_plan_destroy(cp.chunk);
+        if (cp.tail) tfft_plan_destroy(cp.tail);
+    }
     for (void* q : p->allocs) cudaFree(q);
     if (p->status_host) cudaFreeHost(p->status_host);
     delete p;
