@@ -147,6 +147,9 @@ template <> __device__ __forceinline__ float2 acc_zero<float2>() { return make_f
 // FT kernels, which read their weights for every tile.  Before -> after (complex64, sustained): 2^20 x 256 1638 -> 1610 us,
 // 2^21 x 128 1817 -> 1766, 2^20 x 256 with detection 1786 -> 1752, with correction 1805 -> 1770, 2^12 x 2^14 with
 // detection 209.3 -> 206.9; lines of 256 and 512 points do not change.
+// Lines of one register stage read no table that the hint would protect, and each of the two stores of a 2-point line
+// fills half of every 32-byte sector it touches.  1 GiB of such lines with the hint and without: complex64 356 and 324 us,
+// complex128 338 and 311, complex128 with a repair in every block 746 and 642.
 __device__ __forceinline__ void store_result(float2* p, float2 v) {
     asm volatile("st.global.L1::no_allocate.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
 }
@@ -538,6 +541,7 @@ struct Fft {
             for (int i = 0; i < E; ++i) {
                 if (!in_range(a, o0 + (long long)i * TPL * g.out_rs, 4)) continue;
                 if (CS == 2) dst[(long long)i * TPL * g.out_rs] = csub(dst[(long long)i * TPL * g.out_rs], y[i]);
+                else if constexpr (K::S == 1) dst[(long long)i * TPL * g.out_rs] = y[i];
                 else store_result(dst + (long long)i * TPL * g.out_rs, y[i]);
             }
         }
