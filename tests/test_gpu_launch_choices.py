@@ -148,3 +148,29 @@ def test_status_counts_come_from_the_last_exec(torch_cuda, dtype):
     plan.set_injection(False)
     plan(x)
     assert plan.ft_status()[:2] == (0, 0)
+
+
+# small tiles (1 to 2 KB, a tile per block): the last count that overlaps the launch before and the first that does not
+@pytest.mark.parametrize("dtype,logn,inner", [(0, 3, 32), (0, 4, 4), (0, 6, 4), (0, 8, 1), (1, 4, 4), (1, 5, 1)])
+def test_many_small_tiles_along_a_strided_axis(torch_cuda, dtype, logn, inner):
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    n = 1 << logn
+    x = torch.from_numpy(orc.make_input(4097 * inner, n, CD[dtype], seed=logn)).cuda().view(4097, n, inner)
+    want = torch.fft.fft(x.to(torch.complex128), dim=1)
+    few, many = tf.fft(x[:4096], dim=1), tf.fft(x, dim=1)
+    assert _same(torch, few, many[:4096])
+    assert float(torch.linalg.vector_norm(many - want) / torch.linalg.vector_norm(want)) <= orc.tolerance(CD[dtype], logn)
+    # launches of either kind, and of the kernels between, read what the one before wrote
+    def step(v):
+        v = tf.ifft(tf.fft(v, dim=1), dim=1)
+        return tf.fft(v, dim=2, norm="ortho") if inner > 1 else v
+
+    y = z = x
+    for _ in range(6):
+        y = step(y)
+        torch.cuda.synchronize()
+    for _ in range(6):
+        z = step(z)
+    assert _same(torch, y, z)

@@ -100,6 +100,7 @@ struct LaunchDesc {
     int run_logc = 0;
     long long run_tiles = 0;
     unsigned run_grid = 0;
+    bool run_many = false;  // so many small tiles that the kernel without launch overlap is faster (kSmallTile)
     int log_b = 0, log_n1 = 0, log_q = 0, tw_lo_bits = 0;
     void* tw_st = nullptr;
     void* tw_lo = nullptr;
@@ -385,6 +386,7 @@ void adjust_tiles(tfft_plan p) {
             d.run_tiles *= 2;
             d.run_grid = (unsigned)d.run_tiles;
         }
+        d.run_many = d.run_k->fn_many && d.run_grid > kManyBlocks;
     }
 }
 
@@ -414,7 +416,7 @@ constexpr size_t kStatusBytes = 64u << 10;
 // Launches one fft_kernel with the programmatic-dependent-launch attribute (fft_kernels.cuh,
 // wait_for_previous_launch): its blocks are placed while the launch before it drains, where the
 // kernel is built for that.
-cudaError_t launch_kernel(const void* fn, unsigned grid, int threads, void** args, size_t smem, cudaStream_t st, int logm) {
+cudaError_t launch_kernel(const void* fn, unsigned grid, int threads, void** args, size_t smem, cudaStream_t st, bool overlap) {
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -424,7 +426,7 @@ cudaError_t launch_kernel(const void* fn, unsigned grid, int threads, void** arg
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = &attr;
-    cfg.numAttrs = dependent_launch(logm) ? 1 : 0;
+    cfg.numAttrs = overlap ? 1 : 0;
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
@@ -554,9 +556,9 @@ int launch_all(tfft_plan p, const void* in, void* out, cudaStream_t st, void* sc
         a.ft_diag = p->diag ? (T*)d.ft_diag : nullptr;
         void* args[] = {&a};
         const bool use_csum = ftmode == FT_CORRECT && p->csum && csum_ok(d.k);
-        const void* fn = use_csum ? d.k->fn[FT_CSUM] : d.run_k->fn[ftmode];
+        const void* fn = use_csum ? d.k->fn[FT_CSUM] : (d.run_many ? d.run_k->fn_many : d.run_k->fn[ftmode]);
         const size_t smem = use_csum ? d.k->smem_csum : d.run_k->smem;
-        if (!cuda_ok(p, launch_kernel(fn, d.run_grid, d.run_k->threads, args, smem, st, d.logm)))
+        if (!cuda_ok(p, launch_kernel(fn, d.run_grid, d.run_k->threads, args, smem, st, dependent_launch(d.logm) && !d.run_many)))
             return TFFT_ERR_CUDA;
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }
@@ -1507,7 +1509,7 @@ int static_launch(const StaticDeviceState& st, int logN, const void* in, void* o
         a.tw_lo_bits = d.tw_lo_bits;
         a.inj_period = 1;
         void* args[] = {&a};
-        if (launch_kernel(d.k->fn[FT_OFF], d.grid, d.k->threads, args, d.k->smem, stream, d.logm) != cudaSuccess)
+        if (launch_kernel(d.k->fn[FT_OFF], d.grid, d.k->threads, args, d.k->smem, stream, dependent_launch(d.logm)) != cudaSuccess)
             return TFFT_ERR_CUDA;
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }

@@ -166,8 +166,15 @@ __device__ __forceinline__ void store_result(double2* p, double2 v) {
 // 2^16 x 1 10.9 -> 6.0 us, 2^22 x 1 41 -> 34 us, 2^16 x 512 175 -> 170 us (complex64).  The start signal stands before
 // the stores because a launch placed earlier finds the SMs still occupied and is spread unevenly: with the signal at
 // the top of the kernel 2^16 x 8 takes 9.6 us, here 7.1 us.
-// Not for lines of 2 and 4 points, whose launches are hundreds of thousands of blocks of a few KB: there the two
-// instructions cost each block more than the launch gains (2^2 complex64, 1 GiB: 542 us with them, 327 without).
+// A kernel that holds these two instructions starts a block in 1.03 ns, one without in 0.51, with or without the attribute
+// (2^18 blocks of 1 to 2 KB, back to back: 273 us against 140 to 162).  A block that moves less than HBM does in that time is
+// held up by it: tiles under 4 KB (each is read and written).  So the kernels of 2- and 4-point signals have none (1 GiB of
+// 4-point complex64 lines: 547 us with, 330 without), and those of other small tiles, which the strided-batch plans run, exist in
+// both forms: launches of more than kManyBlocks blocks take the one without (capi.cu, run_many).  8-point complex64
+// lines of 2 KB tiles: 2^12 blocks 5.5 us with and 6.2 without, 2^13 9.8 and 8.2, 2^18 273 and 158; from 4 KB on (8-point complex64
+// signals) every count is faster with them, 2^18 blocks by 2 us of 334.
+constexpr int kSmallTile = 4096;
+constexpr unsigned kManyBlocks = 4096;
 __host__ __device__ constexpr bool dependent_launch(int logm) { return logm > 2; }
 __device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;"); }
@@ -305,6 +312,7 @@ struct Cfg {
     // Bound: HBM.  32-point complex64 lines in one thread each (1 GiB): 369 us as four threads of 8 points, whose loads
     // touch a 128-byte line per 32 bytes (343 us with those staged as well), 311 us in this form.
     static constexpr bool STAGED_IO = (ROLE == ROLE_SINGLE && S == 1 && TPL == 1 && LOGM >= 2);
+    static constexpr size_t TILE_BYTES = (size_t)M * C * 2 * sizeof(T);
     static constexpr int SMEM_ELEMS = STAGED_IO ? (M + 1) * C : (S > 1 ? (LAYOUT_COLS ? MPAD * C : PITCH * C) : 0);
     static constexpr size_t SMEM_BYTES = (size_t)SMEM_ELEMS * 2 * sizeof(T);
     // FT_CSUM keeps two more tiles in shared memory: the running sums of inputs and outputs
@@ -325,7 +333,7 @@ struct Cfg {
     }
 };
 
-template <typename T, int LOGM, int LOGE, int LOGC, int ROLE, int FT>
+template <typename T, int LOGM, int LOGE, int LOGC, int ROLE, int FT, bool OVERLAP = dependent_launch(LOGM)>
 struct Fft {
     typedef Cfg<T, LOGM, LOGE, LOGC, ROLE> K;
     typedef typename Cplx<T>::type C;
@@ -521,7 +529,7 @@ struct Fft {
                 y[i].y *= a.scale_y;
             }
         }
-        if constexpr (dependent_launch(LOGM)) let_next_launch_start();
+        if constexpr (OVERLAP) let_next_launch_start();
         if constexpr (K::STAGED_IO && CS != 2) {
             // every thread only touches its own line here, so no barrier is needed before
 #pragma unroll
@@ -816,14 +824,14 @@ struct Fft {
     }
 };
 
-template <typename T, int LOGM, int LOGE, int LOGC, int ROLE, int FT>
+template <typename T, int LOGM, int LOGE, int LOGC, int ROLE, int FT, bool OVERLAP = dependent_launch(LOGM)>
 __global__ void __launch_bounds__((Cfg<T, LOGM, LOGE, LOGC, ROLE>::THREADS),
                                   (Cfg<T, LOGM, LOGE, LOGC, ROLE>::min_blocks(FT)))
 fft_kernel(const __grid_constant__ KernelArgs<T> a) {
     extern __shared__ __align__(16) unsigned char tfft_smem_raw[];
     typedef typename Cplx<T>::type C;
-    if constexpr (dependent_launch(LOGM)) wait_for_previous_launch();
-    Fft<T, LOGM, LOGE, LOGC, ROLE, FT>::run(a, reinterpret_cast<C*>(tfft_smem_raw));
+    if constexpr (OVERLAP) wait_for_previous_launch();
+    Fft<T, LOGM, LOGE, LOGC, ROLE, FT, OVERLAP>::run(a, reinterpret_cast<C*>(tfft_smem_raw));
 }
 
 }  // namespace tfft

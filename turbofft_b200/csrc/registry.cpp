@@ -13,9 +13,10 @@ static std::map<Key, KernelEntry>& table() {
 }
 
 void register_kernel(int dtype, int role, int logm, int loge, int logc, int ft, const void* fn, int threads,
-                     size_t smem, int remlast) {
+                     size_t smem, int remlast, const void* fn_many) {
     KernelEntry& e = table()[Key(dtype, role, logm, loge, logc)];
     e.fn[ft] = fn;
+    if (ft == 0) e.fn_many = fn_many;
     e.threads = threads;
     e.remlast = remlast;
     if (ft == 3) e.smem_csum = smem;

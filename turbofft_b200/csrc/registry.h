@@ -10,6 +10,7 @@ namespace tfft {
 
 struct KernelEntry {
     const void* fn[4];  // FT_OFF, FT_DETECT, FT_CORRECT, FT_CSUM (null = not compiled)
+    const void* fn_many;  // FT_OFF without launch overlap, for launches of very many small tiles (null = fn[FT_OFF] serves)
     int threads;
     size_t smem;        // dynamic shared memory of the first three modes
     size_t smem_csum;   // FT_CSUM adds two tiles of running sums
@@ -17,7 +18,7 @@ struct KernelEntry {
 };
 
 void register_kernel(int dtype, int role, int logm, int loge, int logc, int ft, const void* fn, int threads,
-                     size_t smem, int remlast);
+                     size_t smem, int remlast, const void* fn_many);
 const KernelEntry* find_kernel(int dtype, int role, int logm, int loge, int logc);
 int registered_kernel_count();
 // counts one kernel launch of this library (see tfft_launch_count)
