@@ -150,6 +150,8 @@ template <> __device__ __forceinline__ float2 acc_zero<float2>() { return make_f
 // Lines of one register stage read no table that the hint would protect, and each of the two stores of a 2-point line
 // fills half of every 32-byte sector it touches.  1 GiB of such lines with the hint and without: complex64 356 and 324 us,
 // complex128 338 and 311, complex128 with a repair in every block 746 and 642.
+// Strided complex128 lines of 1024 points (64 KB tiles, two blocks per SM) are the one exchange kernel that loses by it:
+// [32][1024][1024] 245 us with the hint, 238 without; lines of 512, 2048 and 4096 points gain 1 to 7 %.
 __device__ __forceinline__ void store_result(float2* p, float2 v) {
     asm volatile("st.global.L1::no_allocate.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
 }
@@ -312,6 +314,8 @@ struct Cfg {
     // Bound: HBM.  32-point complex64 lines in one thread each (1 GiB): 369 us as four threads of 8 points, whose loads
     // touch a 128-byte line per 32 bytes (343 us with those staged as well), 311 us in this form.
     static constexpr bool STAGED_IO = (ROLE == ROLE_SINGLE && S == 1 && TPL == 1 && LOGM >= 2);
+    // store_result says why
+    static constexpr bool STORE_PAST_L1 = S > 1 && !(ROLE == ROLE_FIRST && sizeof(T) == 8 && LOGM == 10);
     static constexpr size_t TILE_BYTES = (size_t)M * C * 2 * sizeof(T);
     static constexpr int SMEM_ELEMS = STAGED_IO ? (M + 1) * C : (S > 1 ? (LAYOUT_COLS ? MPAD * C : PITCH * C) : 0);
     static constexpr size_t SMEM_BYTES = (size_t)SMEM_ELEMS * 2 * sizeof(T);
@@ -549,7 +553,7 @@ struct Fft {
             for (int i = 0; i < E; ++i) {
                 if (!in_range(a, o0 + (long long)i * TPL * g.out_rs, 4)) continue;
                 if (CS == 2) dst[(long long)i * TPL * g.out_rs] = csub(dst[(long long)i * TPL * g.out_rs], y[i]);
-                else if constexpr (K::S == 1) dst[(long long)i * TPL * g.out_rs] = y[i];
+                else if constexpr (!K::STORE_PAST_L1) dst[(long long)i * TPL * g.out_rs] = y[i];
                 else store_result(dst + (long long)i * TPL * g.out_rs, y[i]);
             }
         }
