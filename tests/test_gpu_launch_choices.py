@@ -174,3 +174,46 @@ def test_many_small_tiles_along_a_strided_axis(torch_cuda, dtype, logn, inner):
     for _ in range(6):
         z = step(z)
     assert _same(torch, y, z)
+
+
+def _located(batch, lines, tbs, n_blocks):
+    """Which tile of each block carries the injected fault, -1 where that tile is beyond the batch."""
+    n_tiles = -(-batch // lines)
+    return [k if (k := orc.injected_tile_iteration(b, tbs)) <= len(orc.b200_block_tiles(b, n_blocks, n_tiles, tbs)) else -1
+            for b in range(n_blocks)]
+
+
+def _check_32_point_plan(torch, plan, batch, if_err, csum):
+    """Output and, with a fault of 1000 in every block, what was located and repaired."""
+    x = orc.make_input(batch, 32, np.complex64, seed=batch)
+    plan.set_ft_params(1000.0, 1000.0, 1e-3)
+    if csum:
+        plan.set_correction(True)
+    y, ref = plan(torch.from_numpy(x).cuda()).cpu().numpy(), orc.fft_forward(x)
+    if csum:
+        # y_bad - (sum of y - F(sum of x)): five stages, the sums over two tiles and the subtraction, each rounded at the
+        # size of the fault, of which a line of the sum holds the results of two
+        assert np.abs(y - ref).max() <= 16 * 2.0**-24 * (1000 + 2 * np.abs(ref).max())
+    else:
+        assert orc.rel_l2(y, ref) <= orc.tolerance(np.complex64, 5)
+    if if_err:
+        nd, nc, located = plan.ft_status()
+        want = _located(batch, plan.info()[0]["lines_per_tile"], 2, len(located))
+        assert located == want and nd == nc == sum(k > 0 for k in want)
+
+
+FT_MODES = [(0, 0, 0), (1, 0, 0), (1, 1, 0), (1, 1, 1)]
+
+
+@pytest.mark.parametrize("if_ft,if_err,csum", FT_MODES)
+@pytest.mark.parametrize("batch", [1, 33, 200])
+def test_a_parameter_file_with_the_row_that_another_replaced(torch_cuda, tmp_path, batch, if_ft, if_err, csum):
+    """32-point complex64 lines as four threads of 8 points, the shipped row until one thread took a whole line."""
+    import turbofft_b200 as tf
+
+    rows = ["0, " * 10 + "0"] + [f"{n}, 1, {n}, 0, 0, 64, 0, 0, {min(1 << n, 16)}, 0, 0" for n in range(1, 5)]
+    path = tmp_path / "param.csv"
+    path.write_text("\n".join(rows + ["5, 1, 5, 0, 0, 32, 0, 0, 8, 0, 0"]) + "\n")
+    plan = tf.Plan(5, batch, 0, if_ft=if_ft, if_err=if_err, thread_bs=2, param_csv=str(path))
+    assert plan.info()[0]["points_per_thread"] == 8 and plan.info()[0]["lines_per_tile"] == 32
+    _check_32_point_plan(torch_cuda, plan, batch, if_err, csum)

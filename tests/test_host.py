@@ -190,3 +190,17 @@ def test_bench_reference_arm_prints_one_json_line():
     d = json.loads(lines[0])
     assert d["impl"] == "reference" and d["unit"] == "GFLOPS" and d["value"] > 0
     assert d["cpu_baseline"]["kind"] == "port" and d["e2e"]["h2d_bytes_per_step"] == 0
+
+
+def test_launches_of_rows_that_were_replaced_stay_compiled():
+    """A caller's own parameter file may hold a row that the shipped table held until another took its place."""
+    import glob
+
+    from turbofft_b200.codegen import fft_codegen
+
+    for dt, kept in fft_codegen.KEPT_LAUNCHES.items():
+        for mode in range(4):
+            text = "".join(open(f).read() for f in glob.glob(os.path.join(ROOT, "turbofft_b200", "csrc", "generated", dt, f"inst_ft{mode}_p*.cu")))
+            ctype, code = ("float", 0) if dt == "float2" else ("double", 1)
+            for logm, loge, logc, role in kept:
+                assert f"TFFT_INST({ctype}, {code}, {logm}, {loge}, {logc}, {role}, {mode})" in text

@@ -29,6 +29,10 @@ sys.path.insert(0, os.path.dirname(PKG))
 from turbofft_b200.planner import launches_of_row, parse_param_csv  # noqa: E402
 from turbofft_b200.codegen import smem_layout  # noqa: E402
 
+# Launches (log2 length, log2 points per thread, log2 lines per tile, role) of rows that a shipped table held until another
+# took their place: a caller's own parameter file may hold them, so they stay compiled in every FT mode.
+KEPT_LAUNCHES = {"float2": [(5, 3, 5, 0)], "double2": []}
+
 PART_SIZE = 6  # instantiations per translation unit (keeps parallel builds balanced)
 
 
@@ -93,6 +97,7 @@ def main(argv=None):
     csv_text = open(os.path.join(pdir, f"param_{args.datatype}.csv")).read()
     rows = parse_param_csv(csv_text)
     inst = collect_instances(rows)
+    inst += [key for key in KEPT_LAUNCHES[args.datatype] if key not in inst]
     extra = os.path.join(pdir, f"extra_{args.datatype}.csv")
     if os.path.exists(extra) and mode == 0:  # tuner candidates are timed with FT off only
         for r in parse_param_csv_multi(open(extra).read()):
