@@ -204,3 +204,49 @@ def test_launches_of_rows_that_were_replaced_stay_compiled():
             ctype, code = ("float", 0) if dt == "float2" else ("double", 1)
             for logm, loge, logc, role in kept:
                 assert f"TFFT_INST({ctype}, {code}, {logm}, {loge}, {logc}, {role}, {mode})" in text
+
+
+def test_library_builds_without_torch(monkeypatch):
+    """The C library and the CLI come before the extension for torch, which is left out where there is none."""
+    from turbofft_b200 import build as b
+
+    done = []
+    monkeypatch.setitem(sys.modules, "torch", None)
+    monkeypatch.setattr(b, "run_codegen", lambda *a: None)
+    monkeypatch.setattr(b, "_objects", lambda sources, *a: (done.append(os.path.basename(sources[0])) or [], True))
+    monkeypatch.setattr(b.subprocess, "run", lambda *a, **k: subprocess.CompletedProcess(a, 0, "", ""))
+    monkeypatch.setattr(b, "TORCH_BINDING", "no such file")
+    build_binding = b.build_torch_binding
+    monkeypatch.setattr(b, "build_torch_binding", lambda *a: (done.append("torch binding"), build_binding(*a)))
+    assert b.build_all(verbose=False) == b.LIB
+    assert done == ["capi.cu", "capi.cu", "cufft_compare.cu", "turbofft_cli.cu", "torch binding"]
+
+
+def test_ft_status_without_torch(monkeypatch):
+    """A program that runs plans on plain pointers reads the status through ctypes alone."""
+    import turbofft_b200 as tf
+
+    class Lib:
+        def tfft_plan_info(self, h, buf):
+            buf[0], buf[4], buf[10] = 2, 3, 5  # two launches of 3 and 5 blocks
+            return 0
+
+        def tfft_ft_status(self, h, nd, nc, launch, loc, cap, nb):
+            assert cap >= 5 and launch in (-1, 0, 1)
+            n = (3, 5)[launch]
+            for i in range(n):
+                loc[i] = 10 * launch + i
+            nd._obj.value, nc._obj.value, nb._obj.value = 7, 6, n
+            return 0
+
+        def tfft_plan_destroy(self, h):
+            return 0
+
+    monkeypatch.setitem(sys.modules, "torch", None)
+    monkeypatch.setattr(tf, "_binding", None)
+    monkeypatch.setattr(tf, "lib", Lib)
+    plan = tf.Plan.__new__(tf.Plan)
+    plan._h = ctypes.c_void_p(1)
+    assert plan.ft_status() == (7, 6, [-10, -9, -8, -7, -6])
+    assert plan.ft_status(0) == (7, 6, [0, 1, 2])
+    plan.destroy()

@@ -187,10 +187,20 @@ class Plan:
 
     def ft_status(self, launch: int = -1):
         """(n_detected, n_corrected, located[list per block of `launch`])."""
-        status = (_binding or _load_binding()).ft_status(self, int(launch))
-        if isinstance(status, int):
-            _lib.check(status, "tfft_ft_status", self._h)
-        return status
+        try:
+            native = _binding or _load_binding()
+        except ImportError:  # no torch: a program that hands over plain pointers (exec_ptr) needs none
+            native = None
+        if native:
+            status = native.ft_status(self, int(launch))
+            if isinstance(status, int):
+                _lib.check(status, "tfft_ft_status", self._h)
+            return status
+        nd, nc, nb = C.c_int(), C.c_int(), C.c_int()
+        most = max(l["grid"] for l in self.info())
+        loc = (C.c_int * most)()
+        _lib.check(lib().tfft_ft_status(self._h, C.byref(nd), C.byref(nc), launch, loc, most, C.byref(nb)), "tfft_ft_status", self._h)
+        return nd.value, nc.value, list(loc[: nb.value])
 
     def ft_diag(self, launch: int = -1):
         """Per block (delta, S, delta_w) of `launch`; needs enable_ft_diag() before exec."""

@@ -5,10 +5,11 @@ passes, then the native build), with nvcc driven directly instead of CMake:
   1. codegen/fft_codegen.py, three passes per datatype (plain, --if_ft 1,
      --if_ft 1 --if_err_injection 1)
   2. every translation unit -> csrc/build/*.o, in parallel
-  3. _torch_binding.so, the native form of the Python call path (ATen, no CUDA code)
-  4. libturbofft_b200.so (the product: kernels + C ABI, no cuFFT),
+  3. libturbofft_b200.so (the product: kernels + C ABI, no cuFFT),
      libturbofft_cufft_cmp.so (cuFFT timing wrapper, comparison only) and the
      `turbofft` command-line driver.
+  4. where torch is installed, _torch_binding.so, the native form of the Python call path
+     (ATen, no CUDA code)
 Objects are rebuilt only when their sources or any header changed.
 """
 from __future__ import annotations
@@ -96,14 +97,19 @@ TORCH_BINDING = os.path.join(PKG, "_torch_binding.so")
 
 
 def build_torch_binding(verbose: bool = True) -> None:
-    """csrc/torch_binding.cpp against the headers of the torch that will load it."""
+    """csrc/torch_binding.cpp against the headers of the torch that will load it.  Without torch there is
+    nothing to build it against and no tensor to call it with; the library and the CLI need neither."""
     src = os.path.join(CSRC, "torch_binding.cpp")
     if os.path.exists(TORCH_BINDING) and os.path.getmtime(TORCH_BINDING) >= os.path.getmtime(src):
         return
     import sysconfig
 
-    import torch
-
+    try:
+        import torch
+    except ImportError:
+        if verbose:
+            print("[build] no torch here: the library is built without the Python call path's extension")
+        return
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc())))
     cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
@@ -120,7 +126,6 @@ def build_torch_binding(verbose: bool = True) -> None:
 def build_all(verbose: bool = True, jobs: int | None = None, with_cli: bool = True) -> str:
     jobs = jobs or max(1, os.cpu_count() or 1)
     run_codegen(verbose)
-    build_torch_binding(verbose)
     gen = sorted(glob.glob(os.path.join(CSRC, "generated", "*", "inst_*.cu")))
     core = [os.path.join(CSRC, f) for f in ("capi.cu", "aux_kernels.cu", "cluster_fft.cu", "pair_fft.cu", "multi_gpu.cu", "registry.cpp", "params.cpp")]
     objs, changed = _objects(core + gen, jobs, verbose)
@@ -160,6 +165,7 @@ def build_all(verbose: bool = True, jobs: int | None = None, with_cli: bool = Tr
                 raise RuntimeError(f"link failed:\n{res.stderr}")
             if verbose:
                 print(f"[build] linked {CLI}")
+    build_torch_binding(verbose)
     return LIB
 
 
