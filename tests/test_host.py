@@ -250,3 +250,28 @@ def test_ft_status_without_torch(monkeypatch):
     assert plan.ft_status() == (7, 6, [-10, -9, -8, -7, -6])
     assert plan.ft_status(0) == (7, 6, [0, 1, 2])
     plan.destroy()
+
+
+def test_extension_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
+    import torch
+
+    from turbofft_b200 import build as b
+
+    built = []
+
+    def compile_it(cmd, **k):
+        built.append(cmd)
+        (tmp_path / "x.so").write_text("")
+        return subprocess.CompletedProcess(cmd, 0, "", "")
+
+    monkeypatch.setattr(b, "TORCH_BINDING", str(tmp_path / "x.so"))
+    monkeypatch.setattr(b, "OBJ", str(tmp_path))
+    monkeypatch.setattr(b, "TORCH_BINDING_STAMP", str(tmp_path / "stamp"), raising=False)
+    monkeypatch.setattr(b.subprocess, "run", compile_it)
+    for _ in range(2):
+        b.build_torch_binding(verbose=False)
+    assert len(built) == 1
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + ".other")
+    for _ in range(2):
+        b.build_torch_binding(verbose=False)
+    assert len(built) == 2

@@ -94,14 +94,13 @@ def _objects(sources, jobs: int, verbose: bool, extra=(), suffix: str = ""):
 
 
 TORCH_BINDING = os.path.join(PKG, "_torch_binding.so")
+TORCH_BINDING_STAMP = os.path.join(OBJ, "torch_binding.txt")  # what the file beside it was built with
 
 
 def build_torch_binding(verbose: bool = True) -> None:
     """csrc/torch_binding.cpp against the headers of the torch that will load it.  Without torch there is
     nothing to build it against and no tensor to call it with; the library and the CLI need neither."""
     src = os.path.join(CSRC, "torch_binding.cpp")
-    if os.path.exists(TORCH_BINDING) and os.path.getmtime(TORCH_BINDING) >= os.path.getmtime(src):
-        return
     import sysconfig
 
     try:
@@ -116,9 +115,17 @@ def build_torch_binding(verbose: bool = True) -> None:
            "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
            "-I" + os.path.join(cuda, "include"), "-I" + sysconfig.get_paths()["include"], src, "-o", TORCH_BINDING,
            "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-ltorch"]
+    # another torch at the same place has other headers and another ABI behind the same command
+    stamp = "\n".join([torch.__version__, torch.version.git_version or "", sys.version] + cmd) + "\n"
+    if os.path.exists(TORCH_BINDING) and os.path.getmtime(TORCH_BINDING) >= os.path.getmtime(src) \
+            and os.path.exists(TORCH_BINDING_STAMP) and open(TORCH_BINDING_STAMP).read() == stamp:
+        return
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"g++ failed on {src}:\n{res.stderr}")
+    os.makedirs(OBJ, exist_ok=True)
+    with open(TORCH_BINDING_STAMP, "w") as f:
+        f.write(stamp)
     if verbose:
         print(f"[build] linked {TORCH_BINDING}")
 
