@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from oracle import fft_oracle as orc
+from turbofft_b200 import planner
 
 pytestmark = pytest.mark.gpu
 
@@ -14,8 +15,9 @@ def _same(torch, a, b):
     return torch.equal(torch.view_as_real(a), torch.view_as_real(b))
 
 
-# smallest and largest two-launch sizes, a three-launch size (complex128 2^20), batches around the 128 and 512 tile limits
-@pytest.mark.parametrize("dtype,logn", [(0, 15), (0, 16), (0, 18), (0, 20), (0, 21), (1, 13), (1, 16), (1, 17), (1, 20)])
+# every size with narrower kernels: two launches, and three (complex128 2^20); batches around the 128 and 512 tile limits; the
+# next sizes, where one signal has tiles enough
+@pytest.mark.parametrize("dtype,logn", [(0, n) for n in range(15, 22)] + [(1, n) for n in range(13, 22)])
 @pytest.mark.parametrize("batch", [1, 2, 5, 16, 33])
 def test_narrow_tiles_give_the_bits_of_wide_ones(torch_cuda, dtype, logn, batch):
     import turbofft_b200 as tf
@@ -24,12 +26,19 @@ def test_narrow_tiles_give_the_bits_of_wide_ones(torch_cuda, dtype, logn, batch)
     if batch << logn > 1 << 22:
         batch = max(1, (1 << 22) >> logn) + 1  # largest batch worth its time, odd
     x = torch.from_numpy(orc.make_input(batch, 1 << logn, CD[dtype], seed=logn + batch)).cuda()
-    y = tf.Plan(logn, batch, dtype)(x)
+    small = tf.Plan(logn, batch, dtype)
+    y = small(x)
     wide = max(batch, min(600, (1 << 25) >> logn))  # enough tiles for the row's own tiles in every launch
     xw = torch.zeros(wide, 1 << logn, dtype=x.dtype, device="cuda")
     xw[:batch] = x
-    yw = tf.Plan(logn, wide, dtype)(xw)
+    large = tf.Plan(logn, wide, dtype)
+    yw = large(xw)
     assert _same(torch, y, yw[:batch])
+    # the plans did run different kernels: the row's own tiles, and in some launch narrower ones
+    own = [1 << l.logc for l in planner.launches_of_row(planner.load_params(("float2", "double2")[dtype], "B200")[logn])]
+    few, many = ([l["lines_per_tile"] for l in p.info()] for p in (small, large))
+    assert many == own
+    assert all(f <= o for f, o in zip(few, own)) and (batch > 1 or (few == own) == (logn >= 20 + dtype))
     assert orc.rel_l2(y[-1:].cpu().numpy(), orc.fft_forward(x[-1:].cpu().numpy())) <= orc.tolerance(CD[dtype], logn)
 
 
@@ -217,3 +226,93 @@ def test_a_parameter_file_with_the_row_that_another_replaced(torch_cuda, tmp_pat
     plan = tf.Plan(5, batch, 0, if_ft=if_ft, if_err=if_err, thread_bs=2, param_csv=str(path))
     assert plan.info()[0]["points_per_thread"] == 8 and plan.info()[0]["lines_per_tile"] == 32
     _check_32_point_plan(torch_cuda, plan, batch, if_err, csum)
+
+
+@pytest.mark.parametrize("if_ft,if_err,csum", FT_MODES)
+@pytest.mark.parametrize("batch", [1, 64, 65, 128, 129, 1000])
+def test_faults_in_staged_32_point_lines(torch_cuda, batch, if_ft, if_err, csum):
+    """The shipped row, one thread per line staged through shared memory: location, repair by recomputing and from the
+    checksums."""
+    import turbofft_b200 as tf
+
+    plan = tf.Plan(5, batch, 0, if_ft=if_ft, if_err=if_err, thread_bs=2)
+    assert plan.info()[0]["points_per_thread"] == 32
+    _check_32_point_plan(torch_cuda, plan, batch, if_err, csum)
+
+
+# lengths with a kernel of half the columns per tile
+@pytest.mark.parametrize("dtype,logn", [(0, 8), (0, 9), (0, 10), (1, 6), (1, 7), (1, 8), (1, 9)])
+def test_narrow_strided_tiles_give_the_bits_of_wide_ones(torch_cuda, dtype, logn):
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    outer = 1 << 14 >> logn  # 512 tiles and more of 4 columns
+    x = torch.from_numpy(orc.make_input(outer * 128, 1 << logn, CD[dtype], seed=logn)).cuda().view(outer, 1 << logn, 128)
+    y, y1 = tf.fft(x, dim=1), tf.fft(x[:1], dim=1)
+    lines = [tf._plan_cache[("strided", 0, logn, 128, o, dtype, False, 0.0)].info()[0]["lines_per_tile"] for o in (outer, 1)]
+    assert lines[1] < lines[0]
+    assert _same(torch, y1, y[:1])
+    want = torch.fft.fft(x.to(torch.complex128), dim=1)
+    assert float(torch.linalg.vector_norm(y - want) / torch.linalg.vector_norm(want)) <= orc.tolerance(CD[dtype], logn)
+
+
+CHAIN = [(2, 5000), (5, 700), (12, 3), (16, 2), (16, 600), (22, 1)]
+
+
+def _round_trips(torch, tf, logn, batch, dtype):
+    """Plans and a step of launches that each read what the one before wrote, in place and out of place, with another
+    library's kernel among them."""
+    fwd, bwd = tf.Plan(logn, batch, dtype), tf.Plan(logn, batch, dtype)
+    bwd.set_direction(True, 1.0 / (1 << logn))
+
+    def step(y, z):
+        fwd(y, z)
+        bwd(z, z)
+        fwd(z, y)
+        z.copy_(y)
+        bwd(z, y)
+
+    x = torch.from_numpy(orc.make_input(batch, 1 << logn, CD[dtype], seed=6)).cuda()
+    want, z = x.clone(), torch.empty_like(x)
+    for _ in range(4):
+        step(want, z)
+        torch.cuda.synchronize()
+    return fwd, bwd, step, x, want
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("logn,batch", CHAIN)
+def test_a_captured_chain_of_launches(torch_cuda, logn, batch, dtype):
+    """Overlapped launches become programmatic edges of a graph; replayed twice on the same buffers."""
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    _, _, step, x, want = _round_trips(torch, tf, logn, batch, dtype)
+    y, z = x.clone(), torch.empty_like(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step(y, z)
+        step(y, z)
+    y.copy_(x)
+    graph.replay()
+    graph.replay()
+    assert _same(torch, y, want)
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("logn,batch", CHAIN)
+def test_a_chain_of_launches_across_two_streams(torch_cuda, logn, batch, dtype):
+    """An event between two streams orders the whole of what an exec wrote, not only the blocks that had started."""
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    _, _, step, x, want = _round_trips(torch, tf, logn, batch, dtype)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    y, z = x.clone(), torch.empty_like(x)
+    streams[0].wait_stream(torch.cuda.current_stream())
+    for i in range(4):
+        with torch.cuda.stream(streams[i % 2]):
+            step(y, z)
+        streams[1 - i % 2].wait_stream(streams[i % 2])
+    torch.cuda.synchronize()
+    assert _same(torch, y, want)
