@@ -194,3 +194,26 @@ def test_whole_numbers_beyond_a_machine_word(torch_cuda):
     plan(x)
     assert plan.ft_status(1 << 70) == plan.ft_status(0) == plan.ft_status()
     assert plan.ft_status((1 << 70) - 1) == plan.ft_status(-1)
+
+
+@pytest.mark.parametrize("make", ["plain", "multi", "ft", "strided", "single_pass"])
+def test_making_a_plan_waits_for_nothing_the_caller_has_queued(torch_cuda, make):
+    import turbofft_b200 as tf
+
+    torch = torch_cuda
+    x = torch.zeros(64, 8, 16, dtype=torch.complex64, device="cuda")
+
+    def new(batch):
+        if make == "strided":
+            return tf.fft(torch.zeros(batch, 8, 16, dtype=torch.complex64, device="cuda"), dim=1)
+        if make == "single_pass":
+            return tf.Plan(15, batch, 0, single_pass=-1)
+        return tf.Plan(18 if make == "multi" else 10, batch, 0, if_ft=int(make == "ft"))
+
+    kept = [new(61)]  # the first of its kind loads its kernels, which may wait
+    torch.cuda.synchronize()
+    x.add_(1)
+    torch.cuda._sleep(400_000_000)  # a fifth of a second on the default stream
+    kept.append(new(62))
+    assert not torch.cuda.default_stream().query()
+    torch.cuda.synchronize()
