@@ -124,75 +124,85 @@ PyObject* make_key(PyObject* const* a, const KeyFields& f, int64_t outer, int co
     return key;
 }
 
+// torch's own translation, without the buffer for warnings that its macro sets up on every call
+PyObject* raise_as_torch_does() {
+    torch::translate_exception_to_python(std::current_exception());
+    return nullptr;
+}
+
 // fft(x, ft, err, thread_bs, out, norm_exponent, inverse, dim): the transform along one axis, or None
 PyObject* fast_fft(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
-    if (n != 8 || !g_exec || !ordinary(a[0]) || !PyLong_Check(a[7])) Py_RETURN_NONE;
-    const at::Tensor& x = THPVariable_Unpack(a[0]);
-    const int code = type_code(x);
-    const int64_t rank = x.dim();
-    int overflow = 0;  // the Python path takes an axis of any size modulo the rank
-    int64_t dim = PyLong_AsLongLongAndOverflow(a[7], &overflow);
-    if (overflow) Py_RETURN_NONE;
-    if (dim < 0) dim += rank;
-    if (code < 0 || !x.is_cuda() || dim < 0 || dim >= rank || x.numel() == 0 || !x.is_contiguous()) Py_RETURN_NONE;
-    const int64_t len = x.size(dim);
-    if (len < 2 || (len & (len - 1))) Py_RETURN_NONE;
-    const int logn = __builtin_ctzll((unsigned long long)len);
-    if (a[4] != Py_None) {
-        if (!ordinary(a[4])) Py_RETURN_NONE;
-        const at::Tensor& y = THPVariable_Unpack(a[4]);
-        if (!y.is_cuda() || !y.is_contiguous() || y.scalar_type() != x.scalar_type() || y.sizes() != x.sizes()) Py_RETURN_NONE;
+    try {
+        if (n != 8 || !g_exec || !ordinary(a[0]) || !PyLong_Check(a[7])) Py_RETURN_NONE;
+        const at::Tensor& x = THPVariable_Unpack(a[0]);
+        const int code = type_code(x);
+        const int64_t rank = x.dim();
+        int overflow = 0;  // the Python path takes an axis of any size modulo the rank
+        int64_t dim = PyLong_AsLongLongAndOverflow(a[7], &overflow);
+        if (overflow) Py_RETURN_NONE;
+        if (dim < 0) dim += rank;
+        if (code < 0 || !x.is_cuda() || dim < 0 || dim >= rank || x.numel() == 0 || !x.is_contiguous()) Py_RETURN_NONE;
+        const int64_t len = x.size(dim);
+        if (len < 2 || (len & (len - 1))) Py_RETURN_NONE;
+        const int logn = __builtin_ctzll((unsigned long long)len);
+        if (a[4] != Py_None) {
+            if (!ordinary(a[4])) Py_RETURN_NONE;
+            const at::Tensor& y = THPVariable_Unpack(a[4]);
+            if (!y.is_cuda() || !y.is_contiguous() || y.scalar_type() != x.scalar_type() || y.sizes() != x.sizes()) Py_RETURN_NONE;
+        }
+        const int ft = PyObject_IsTrue(a[1]), err = PyObject_IsTrue(a[2]), inverse = PyObject_IsTrue(a[6]);
+        if (ft < 0 || err < 0 || inverse < 0) return nullptr;
+        const bool strided = dim != rank - 1;
+        if (strided && (ft || err || a[4] != Py_None)) Py_RETURN_NONE;
+        int64_t inner = 1;
+        for (int64_t d = dim + 1; d < rank; ++d) inner *= x.size(d);
+        // a program repeats a handful of shapes: their key tuples are kept, the plans stay the dictionary's
+        const int64_t thread_bs = PyLong_Check(a[3]) ? PyLong_AsLongLong(a[3]) : -1;
+        const double expo = PyFloat_Check(a[5]) ? PyFloat_AS_DOUBLE(a[5]) : 2.0;
+        if (thread_bs < 0 || expo > 1.0) {
+            PyErr_Clear();
+            Py_RETURN_NONE;
+        }
+        const KeyFields fields = {x.device().index(), logn, x.numel() / len, strided ? inner : 0, thread_bs, expo,
+                                  code | ft << 1 | err << 2 | inverse << 3};
+        KeySlot& slot = g_keys[(fields.batch * 31 + fields.logn * 7 + fields.flags) & (kKeySlots - 1)];
+        PyObject* key = slot.key && slot.fields == fields ? slot.key : nullptr;
+        if (!key) key = make_key(a, fields, x.numel() / (len * inner), code, ft, err, inverse, slot);
+        if (!key) return nullptr;
+        PyObject* found = PyDict_GetItemWithError(g_plans, key);  // borrowed
+        if (!found) {
+            if (PyErr_Occurred()) return nullptr;
+            Py_RETURN_NONE;
+        }
+        Py_INCREF(found);
+        THPObjectPtr plan(found);  // held while the interpreter lock is released
+        void* h = plan_handle(found);
+        if (!h) Py_RETURN_NONE;
+        return execute(h, true, x, a[4]);
+    } catch (...) {
+        return raise_as_torch_does();
     }
-    const int ft = PyObject_IsTrue(a[1]), err = PyObject_IsTrue(a[2]), inverse = PyObject_IsTrue(a[6]);
-    if (ft < 0 || err < 0 || inverse < 0) return nullptr;
-    const bool strided = dim != rank - 1;
-    if (strided && (ft || err || a[4] != Py_None)) Py_RETURN_NONE;
-    int64_t inner = 1;
-    for (int64_t d = dim + 1; d < rank; ++d) inner *= x.size(d);
-    // a program repeats a handful of shapes: their key tuples are kept, the plans stay the dictionary's
-    const int64_t thread_bs = PyLong_Check(a[3]) ? PyLong_AsLongLong(a[3]) : -1;
-    const double expo = PyFloat_Check(a[5]) ? PyFloat_AS_DOUBLE(a[5]) : 2.0;
-    if (thread_bs < 0 || expo > 1.0) {
-        PyErr_Clear();
-        Py_RETURN_NONE;
-    }
-    const KeyFields fields = {x.device().index(), logn, x.numel() / len, strided ? inner : 0, thread_bs, expo,
-                              code | ft << 1 | err << 2 | inverse << 3};
-    KeySlot& slot = g_keys[(fields.batch * 31 + fields.logn * 7 + fields.flags) & (kKeySlots - 1)];
-    PyObject* key = slot.key && slot.fields == fields ? slot.key : nullptr;
-    if (!key) key = make_key(a, fields, x.numel() / (len * inner), code, ft, err, inverse, slot);
-    if (!key) return nullptr;
-    PyObject* found = PyDict_GetItemWithError(g_plans, key);  // borrowed
-    if (!found) {
-        if (PyErr_Occurred()) return nullptr;
-        Py_RETURN_NONE;
-    }
-    Py_INCREF(found);
-    THPObjectPtr plan(found);  // held while the interpreter lock is released
-    void* h = plan_handle(found);
-    if (!h) Py_RETURN_NONE;
-    return execute(h, true, x, a[4]);
-    END_HANDLE_TH_ERRORS
 }
 
 // exec(plan, x, out): Plan.__call__, or None
 PyObject* fast_exec(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
-    if (n != 3 || !g_exec || !ordinary(a[1]) || (a[2] != Py_None && !ordinary(a[2]))) Py_RETURN_NONE;
-    const at::Tensor& x = THPVariable_Unpack(a[1]);
-    void* h = plan_handle(a[0]);
-    int logn, dtype, device;
-    long long batch;
-    if (!h || g_shape(h, &logn, &batch, &dtype, &device) != 0) Py_RETURN_NONE;
-    if (!x.is_cuda() || type_code(x) != dtype || x.numel() != (batch << logn) || x.device().index() != device || !x.is_contiguous())
-        Py_RETURN_NONE;
-    if (a[2] != Py_None) {
-        const at::Tensor& y = THPVariable_Unpack(a[2]);
-        if (!y.is_cuda() || !y.is_contiguous() || y.scalar_type() != x.scalar_type() || y.numel() != x.numel()) Py_RETURN_NONE;
+    try {
+        if (n != 3 || !g_exec || !ordinary(a[1]) || (a[2] != Py_None && !ordinary(a[2]))) Py_RETURN_NONE;
+        const at::Tensor& x = THPVariable_Unpack(a[1]);
+        void* h = plan_handle(a[0]);
+        int logn, dtype, device;
+        long long batch;
+        if (!h || g_shape(h, &logn, &batch, &dtype, &device) != 0) Py_RETURN_NONE;
+        if (!x.is_cuda() || type_code(x) != dtype || x.numel() != (batch << logn) || x.device().index() != device || !x.is_contiguous())
+            Py_RETURN_NONE;
+        if (a[2] != Py_None) {
+            const at::Tensor& y = THPVariable_Unpack(a[2]);
+            if (!y.is_cuda() || !y.is_contiguous() || y.scalar_type() != x.scalar_type() || y.numel() != x.numel()) Py_RETURN_NONE;
+        }
+        return execute(h, false, x, a[2]);
+    } catch (...) {
+        return raise_as_torch_does();
     }
-    return execute(h, false, x, a[2]);
-    END_HANDLE_TH_ERRORS
 }
 
 // ft_status(plan, launch): (detected, corrected, [located per block]) with one library call, or the negative status
