@@ -200,7 +200,7 @@ int tfft_set_direction(tfft_plan plan, int inverse, double scale);
 int tfft_set_injection(tfft_plan plan, int enable, int launch, int period, int phase);
 
 /* FT outcome of the most recent tfft_exec (synchronises the plan's last
- * stream).  n_detected / n_corrected: blocks whose checksum test fired / tiles
+ * stream and the default one, on which a captured exec may have been replayed).  n_detected / n_corrected: blocks whose checksum test fired / tiles
  * recomputed, summed over launches.  located (may be NULL): for launch
  * `launch`, the per-block located tile iteration, 1-based, -1 = nothing
  * detected -- the register `k` of the reference kernels
